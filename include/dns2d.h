@@ -286,9 +286,9 @@ int dns2d_closure_clamp(dns2d_state *s, float alpha);
 
 /* Autotuner (no counterpart in the reference): times the kernel variants of size N on a scratch
  * state on `device` -- rows per CTA and the radix plans of the small-grid (N <= 512) row and
- * column passes, one or two thread groups per column CTA and the L2 prefetch distances of the
- * large-grid passes -- and keeps the fastest for states and batches created afterwards on that
- * device.  Rows per CTA, thread groups and prefetch distances do not change the arithmetic; a
+ * column passes -- and keeps the fastest for states and batches created afterwards on that
+ * device; the larger sizes have one configuration, and cols_groups, pf_rows and pf_cols are
+ * accepted and reported but select nothing.  Rows per CTA do not change the arithmetic; a
  * radix plan changes the FP32 rounding (every plan meets the oracle tolerances), and an
  * alternative plan is kept only when it is at least 3 % faster than the default one.  config
  * (nullable, 6 ints) receives {rows_tile, cols_groups, pf_rows, pf_cols, plan_rows, plan_cols}

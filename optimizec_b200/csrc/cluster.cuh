@@ -113,22 +113,31 @@ struct Peers {
 template <int N>
 __device__ __forceinline__ void cross_fwd(float2 (&x)[4], const Peers &dst, int m, const float2 *tw)
 {
-    DFT<4, false>::run(x);
+    cscalar v[4];
 #pragma unroll
-    for (int r = 1; r < 4; ++r) x[r] = cmul(x[r], cross_tw<N>(tw, r, m));
+    for (int r = 0; r < 4; ++r) v[r] = {x[r].x, x[r].y};
+    DFT<4, false>::run(v);
 #pragma unroll
-    for (int r = 0; r < 4; ++r) dst.p[r][sidx<CfgC<N>::PS>(m)] = x[r];
+    for (int r = 1; r < 4; ++r) v[r] = cmul(v[r], cross_tw<N>(tw, r, m));
+#pragma unroll
+    for (int r = 0; r < 4; ++r) dst.p[r][sidx<CfgC<N>::PS>(m)] = make_float2(v[r].x, v[r].y);
 }
 
 // inverse cluster butterfly for position m: P_c[m] from the 4 CTAs in, x[m + M s] out
 template <int N>
 __device__ __forceinline__ void cross_inv(float2 (&x)[4], const Peers &src, int m, const float2 *tw)
 {
+    cscalar v[4];
 #pragma unroll
-    for (int r = 0; r < 4; ++r) x[r] = src.p[r][sidx<CfgC<N>::PS>(m)];
+    for (int r = 0; r < 4; ++r) {
+        const float2 e = src.p[r][sidx<CfgC<N>::PS>(m)];
+        v[r] = {e.x, e.y};
+    }
 #pragma unroll
-    for (int r = 1; r < 4; ++r) x[r] = cmul(x[r], cconj(cross_tw<N>(tw, r, m)));
-    DFT<4, true>::run(x);
+    for (int r = 1; r < 4; ++r) v[r] = cmul(v[r], cconj(cross_tw<N>(tw, r, m)));
+    DFT<4, true>::run(v);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) x[r] = make_float2(v[r].x, v[r].y);
 }
 
 // Hermitian packing of U + iW (row z) at mode k (C2R semantics: Re only on kx = 0)
@@ -138,7 +147,7 @@ __device__ __forceinline__ float2 packed_uw(const float2 *__restrict__ U, const 
     const bool lo = k < H, hi = k > L - H;
     if (!lo && !hi) return make_float2(0.f, 0.f);
     const int kk = lo ? k : L - k;
-    const float2 a = U[(size_t)kk << 2], b = W[(size_t)kk << 2];
+    const float2 a = U[(size_t)kk * widx_kx_stride], b = W[(size_t)kk * widx_kx_stride];
     if (k == 0) return make_float2(a.x, b.x);
     if (lo) return make_float2(a.x - b.y, a.y + b.x);
     return make_float2(a.x + b.y, b.x - a.y);
@@ -159,8 +168,7 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(CfgC<N>::NT, CfgC<N>
     const int c = (int)cl.block_rank();
     const int z = blockIdx.x >> 2;
     const Peers pe(cl, s);
-    const float2 *__restrict__ U = p.work + widx<L, H>(0, z, 0);
-    const float2 *__restrict__ W = p.work + widx<L, H>(1, z, 0);
+    const float2 *__restrict__ U = p.work + widx<L, H>(0, z, 0);  // W one float2 behind U
     // Q[k] of the Hermitian packing belongs to CTA k % 4 at position k / 4.  Each CTA reads a
     // contiguous quarter of U, W (k < H) once and stores Q[k] and Q[L-k] into the owners' shared
     // memory; the zero band [H, L-H] is cleared locally.  The first barrier makes sure every CTA
@@ -174,7 +182,8 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(CfgC<N>::NT, CfgC<N>
         constexpr int HQ = (H + 3) / 4;
         const int k0 = c * HQ, k1 = min(H, k0 + HQ);
         for (int k = k0 + (int)threadIdx.x; k < k1; k += NT) {
-            const float2 a = U[(size_t)k << 2], b = W[(size_t)k << 2];
+            const float4 uw = *reinterpret_cast<const float4 *>(U + (size_t)k * widx_kx_stride);
+            const float2 a = make_float2(uw.x, uw.y), b = make_float2(uw.z, uw.w);
             if (k == 0) {
                 pe.p[0][sidx<CfgC<N>::PS>(0)] = make_float2(a.x, b.x);
             } else {
@@ -185,7 +194,7 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(CfgC<N>::NT, CfgC<N>
         }
     }
     cl.sync();
-    fft_run<Cat, M, MP, true, 1, NT, CfgC<N>::PS>(s, p.tw, typename C::Plan{});
+    fft_run<Cat, M, MP, true, 1, NT, CfgC<N>::PS, false, cscalar>(s, p.tw, typename C::Plan{});
     cl.sync();
     const int m1 = min(M, (c + 1) * MQ);
     for (int m = c * MQ + threadIdx.x; m < m1; m += NT) {
@@ -196,12 +205,11 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(CfgC<N>::NT, CfgC<N>
         cross_fwd<N>(x, pe, m, p.tw);
     }
     cl.sync();
-    fft_run<Cat, M, MP, false, 1, NT, CfgC<N>::PS>(s, p.tw, typename C::Plan{});
+    fft_run<Cat, M, MP, false, 1, NT, CfgC<N>::PS, false, cscalar>(s, p.tw, typename C::Plan{});
     cl.sync();
     // unpack D = (Q[k] + conj Q[L-k]) / 2, E = -i (Q[k] - conj Q[L-k]) / 4 for k < H; Q[k] sits in
     // CTA k % 4 at position k / 4.  Each CTA writes a contiguous quarter of the k range.
-    float2 *__restrict__ Do = p.work + widx<L, H>(0, z, 0);
-    float2 *__restrict__ Eo = p.work + widx<L, H>(1, z, 0);
+    float2 *__restrict__ Do = p.work + widx<L, H>(0, z, 0);  // E one float2 behind D
     {
         constexpr int HQ = (H + 3) / 4;
         const int k0 = c * HQ, k1 = min(H, k0 + HQ);
@@ -209,8 +217,8 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(CfgC<N>::NT, CfgC<N>
             const int kp = (k == 0) ? 0 : L - k;
             const float2 q = pe.p[k & 3][sidx<CfgC<N>::PS>(k >> 2)];
             const float2 m = pe.p[kp & 3][sidx<CfgC<N>::PS>(kp >> 2)];
-            Do[(size_t)k << 2] = make_float2(0.5f * (q.x + m.x), 0.5f * (q.y - m.y));
-            Eo[(size_t)k << 2] = make_float2(0.25f * (q.y + m.y), -0.25f * (q.x - m.x));
+            *reinterpret_cast<float4 *>(Do + (size_t)k * widx_kx_stride) =
+                make_float4(0.5f * (q.x + m.x), 0.5f * (q.y - m.y), 0.25f * (q.y + m.y), -0.25f * (q.x - m.x));
         }
     }
     cluster_sync_relaxed();
@@ -297,15 +305,16 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(CfgC<N>::NT, CfgC<N>
         float2 d[4], e[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            d[q] = p.work[widx<L, H>(0, m + q * M, kx)];
-            e[q] = p.work[widx<L, H>(1, m + q * M, kx)];
+            const float4 de = *reinterpret_cast<const float4 *>(p.work + widx<L, H>(0, m + q * M, kx));
+            d[q] = make_float2(de.x, de.y);
+            e[q] = make_float2(de.z, de.w);
         }
         cross_fwd<N>(d, pD, m, p.tw);
         cross_fwd<N>(e, pE, m, p.tw);
     }
     cl.sync();
-    fft_run<Cat, M, MP, false, 1, NT, CfgC<N>::PS>(sD, p.tw, typename C::Plan{});
-    fft_run<Cat, M, MP, false, 1, NT, CfgC<N>::PS>(sE, p.tw, typename C::Plan{});
+    fft_run<Cat, M, MP, false, 1, NT, CfgC<N>::PS, false, cscalar>(sD, p.tw, typename C::Plan{});
+    fft_run<Cat, M, MP, false, 1, NT, CfgC<N>::PS, false, cscalar>(sE, p.tw, typename C::Plan{});
 
     const StepParams prm = *p.prm;
     const float dt = prm.dt;
@@ -352,18 +361,17 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(CfgC<N>::NT, CfgC<N>
     ez = block_sum2<NT>(ez, red);
     if (threadIdx.x == 0) cpart = ez;
     __syncthreads();
-    fft_run<Cat, M, MP, true, 1, NT, CfgC<N>::PS>(sD, p.tw, typename C::Plan{});
-    fft_run<Cat, M, MP, true, 1, NT, CfgC<N>::PS>(sE, p.tw, typename C::Plan{});
+    fft_run<Cat, M, MP, true, 1, NT, CfgC<N>::PS, false, cscalar>(sD, p.tw, typename C::Plan{});
+    fft_run<Cat, M, MP, true, 1, NT, CfgC<N>::PS, false, cscalar>(sE, p.tw, typename C::Plan{});
     cl.sync();
     cluster_energy<NT>(cl, p, kx, gridDim.x >> 2, &cpart, red, &am_last, hist_slot);
     for (int m = m0 + threadIdx.x; m < m1; m += NT) {
-        float2 x[4];
+        float2 x[4], y[4];
         cross_inv<N>(x, pD, m, p.tw);
+        cross_inv<N>(y, pE, m, p.tw);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) p.work[widx<L, H>(0, m + q * M, kx)] = x[q];
-        cross_inv<N>(x, pE, m, p.tw);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) p.work[widx<L, H>(1, m + q * M, kx)] = x[q];
+        for (int q = 0; q < 4; ++q)
+            *reinterpret_cast<float4 *>(p.work + widx<L, H>(0, m + q * M, kx)) = make_float4(x[q].x, x[q].y, y[q].x, y[q].y);
     }
     cluster_sync_relaxed();
 }
@@ -408,17 +416,16 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(CfgC<N>::NT, CfgC<N>
         sW[sidx<CfgC<N>::PS>(k2)] = w;
     }
     __syncthreads();
-    fft_run<Cat, M, MP, true, 1, NT, CfgC<N>::PS>(sU, p.tw, typename C::Plan{});
-    fft_run<Cat, M, MP, true, 1, NT, CfgC<N>::PS>(sW, p.tw, typename C::Plan{});
+    fft_run<Cat, M, MP, true, 1, NT, CfgC<N>::PS, false, cscalar>(sU, p.tw, typename C::Plan{});
+    fft_run<Cat, M, MP, true, 1, NT, CfgC<N>::PS, false, cscalar>(sW, p.tw, typename C::Plan{});
     cl.sync();
     for (int m = c * MQ + threadIdx.x; m < min(M, (c + 1) * MQ); m += NT) {
-        float2 x[4];
+        float2 x[4], y[4];
         cross_inv<N>(x, pU, m, p.tw);
+        cross_inv<N>(y, pW, m, p.tw);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) p.work[widx<L, H>(0, m + q * M, kx)] = x[q];
-        cross_inv<N>(x, pW, m, p.tw);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) p.work[widx<L, H>(1, m + q * M, kx)] = x[q];
+        for (int q = 0; q < 4; ++q)
+            *reinterpret_cast<float4 *>(p.work + widx<L, H>(0, m + q * M, kx)) = make_float4(x[q].x, x[q].y, y[q].x, y[q].y);
     }
     cl.sync();
 }
@@ -445,7 +452,7 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(CfgC<N>::NT, CfgC<N>
     const float2 *__restrict__ W = p.work + widx<L, H>(1, z, 0);
     for (int k2 = threadIdx.x; k2 < M; k2 += NT) s[sidx<CfgC<N>::PS>(k2)] = packed_uw<L, H>(U, W, 4 * k2 + c);
     __syncthreads();
-    fft_run<Cat, M, MP, true, 1, NT, CfgC<N>::PS>(s, p.tw, typename C::Plan{});
+    fft_run<Cat, M, MP, true, 1, NT, CfgC<N>::PS, false, cscalar>(s, p.tw, typename C::Plan{});
     cl.sync();
     float mx = 0.0f;
     for (int m = c * MQ + threadIdx.x; m < min(M, (c + 1) * MQ); m += NT) {
@@ -494,7 +501,7 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(CfgC<N>::NT, CfgC<N>
         cross_fwd<N>(x, pe, m, p.tw);
     }
     cl.sync();
-    fft_run<Cat, M, MP, false, 1, NT, CfgC<N>::PS>(s, p.tw, typename C::Plan{});
+    fft_run<Cat, M, MP, false, 1, NT, CfgC<N>::PS, false, cscalar>(s, p.tw, typename C::Plan{});
     cl.sync();
     const float sc = 1.0f / (float)L;
     float2 *__restrict__ Uo = p.work + widx<L, H>(0, z, 0);
@@ -504,8 +511,8 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(CfgC<N>::NT, CfgC<N>
         const int kp = (k == 0) ? 0 : L - k;
         const float2 q = s[sidx<CfgC<N>::PS>(k2)];
         const float2 m = pe.p[kp & 3][sidx<CfgC<N>::PS>(kp >> 2)];
-        Uo[(size_t)k << 2] = make_float2(0.5f * sc * (q.x + m.x), 0.5f * sc * (q.y - m.y));
-        Wo[(size_t)k << 2] = make_float2(0.5f * sc * (q.y + m.y), -0.5f * sc * (q.x - m.x));
+        Uo[(size_t)k * widx_kx_stride] = make_float2(0.5f * sc * (q.x + m.x), 0.5f * sc * (q.y - m.y));
+        Wo[(size_t)k * widx_kx_stride] = make_float2(0.5f * sc * (q.y + m.y), -0.5f * sc * (q.x - m.x));
     }
     cl.sync();
 }
@@ -540,13 +547,13 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(CfgC<N>::NT, CfgC<N>
         s[sidx<CfgC<N>::PS>(k2)] = v;
     }
     __syncthreads();
-    fft_run<Cat, M, MP, true, 1, NT, CfgC<N>::PS>(s, p.tw, typename C::Plan{});
+    fft_run<Cat, M, MP, true, 1, NT, CfgC<N>::PS, false, cscalar>(s, p.tw, typename C::Plan{});
     cl.sync();
     for (int m = c * MQ + threadIdx.x; m < min(M, (c + 1) * MQ); m += NT) {
         float2 x[4];
         cross_inv<N>(x, pe, m, p.tw);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) scratch[widx<L, H>(0, m + q * M, kx)] = x[q];
+        for (int q = 0; q < 4; ++q) scratch[widx1<L, H>(m + q * M, kx)] = x[q];
     }
     cl.sync();
 }
@@ -565,22 +572,22 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(CfgC<N>::NT, CfgC<N>
     const int c = (int)cl.block_rank();
     const int z = blockIdx.x >> 2;
     const Peers pe(cl, s);
-    const float2 *__restrict__ A = scratch + widx<L, H>(0, z, 0);
+    const float2 *__restrict__ A = scratch + widx1<L, H>(z, 0);
     for (int k2 = threadIdx.x; k2 < M; k2 += NT) {
         const int k = 4 * k2 + c;
         float2 v = make_float2(0.f, 0.f);
         if (k == 0) {
             v = make_float2(A[0].x, 0.f);
         } else if (k < H) {
-            v = A[(size_t)k << 2];
+            v = A[(size_t)k * sidx_kx_stride];
         } else if (k > L - H) {
-            const float2 a = A[(size_t)(L - k) << 2];
+            const float2 a = A[(size_t)(L - k) * sidx_kx_stride];
             v = make_float2(a.x, -a.y);
         }
         s[sidx<CfgC<N>::PS>(k2)] = v;
     }
     __syncthreads();
-    fft_run<Cat, M, MP, true, 1, NT, CfgC<N>::PS>(s, p.tw, typename C::Plan{});
+    fft_run<Cat, M, MP, true, 1, NT, CfgC<N>::PS, false, cscalar>(s, p.tw, typename C::Plan{});
     cl.sync();
     float mn = 3.402823466e38f, mx = -3.402823466e38f;
     for (int m = c * MQ + threadIdx.x; m < min(M, (c + 1) * MQ); m += NT) {

@@ -52,7 +52,10 @@ namespace {
 // kernel configuration of one size on one device; every variant computes the same arithmetic,
 // so the choice changes speed only
 struct Tuning {
-    int rows_tile = 0, cols_groups = 0, pf_rows = 296, pf_cols = 74;
+    int rows_tile = 0;
+    // thread groups and prefetch distances of earlier large-grid kernels: accepted and reported
+    // (dns2d_set_tuning, dns2d_autotune), no kernel reads them
+    int cols_groups = 2, pf_rows = 0, pf_cols = 0;
     int plan_rows = 0, plan_cols = 0;  // radix plans (these change the rounding)
 };
 
@@ -70,9 +73,6 @@ Tuning tuning_for(int device, int N)
 void apply_tuning(Pointers &p, const Tuning &t)
 {
     p.rows_tile = t.rows_tile;
-    p.cols_groups = t.cols_groups;
-    p.pf_rows = t.pf_rows;
-    p.pf_cols = t.pf_cols;
     p.plan_rows = t.plan_rows;
     p.plan_cols = t.plan_cols;
 }
@@ -119,8 +119,10 @@ const KernelSet *kernel_set(int N)
     return nullptr;
 }
 
-// sizes served by the 4-CTA cluster kernels (one configuration each: not autotuned)
+// sizes served by the 4-CTA cluster kernels
 bool cluster_size(int N) { return N == 840 || N == 8192 || N == 9216 || N == 16384 || N == 29400; }
+// sizes with one kernel configuration (nothing for the autotuner to choose)
+bool single_config(int N) { return N >= 1024 || cluster_size(N); }
 
 // ============================================================================================
 // small non-templated kernels
@@ -2160,36 +2162,13 @@ extern "C" int dns2d_batch_autotune(dns2d_batch *b)
         return ms / (float)reps;
     };
     for (BatchGroup &g : b->groups) {
-        if (cluster_size(g.N)) continue;
-        const int reps = g.N >= 2048 ? 10 : 50;
-        Tuning best = g.tune;
-        float tb = 1e30f;
-        if (g.N >= 1024) {
-            for (int pf : {0, 148, 296, 444, 592}) {
-                g.tune = best;
-                g.tune.pf_rows = pf;
-                const Pointers p = g.ptrs();
-                const float t = timed([&] { g.ks->rows_step(p, b->stream, g.count); }, reps);
-                if (t < tb) tb = t, best.pf_rows = pf;
-            }
-            tb = 1e30f;
-            for (int gr : {1, 2})
-                for (int pf : {0, 37, 74, 148}) {
-                    g.tune = best;
-                    g.tune.cols_groups = gr;
-                    g.tune.pf_cols = pf;
-                    const Pointers p = g.ptrs();
-                    const float t = timed([&] { g.ks->cols_step(p, 0, 0, b->stream, g.count); }, reps);
-                    if (t < tb) tb = t, best.cols_groups = gr, best.pf_cols = pf;
-                }
-        } else {
-            best = tune_small(g.ks->nplans, best, [&](const Tuning &t, bool rows) {
-                g.tune = t;
-                const Pointers p = g.ptrs();
-                if (rows) return timed([&] { g.ks->rows_step(p, b->stream, g.count); }, reps);
-                return timed([&] { g.ks->cols_step(p, 0, 0, b->stream, g.count); }, reps);
-            });
-        }
+        if (single_config(g.N)) continue;
+        const Tuning best = tune_small(g.ks->nplans, g.tune, [&](const Tuning &t, bool rows) {
+            g.tune = t;
+            const Pointers p = g.ptrs();
+            if (rows) return timed([&] { g.ks->rows_step(p, b->stream, g.count); }, 50);
+            return timed([&] { g.ks->cols_step(p, 0, 0, b->stream, g.count); }, 50);
+        });
         g.tune = best;
     }
     cudaEventDestroy(e0);
@@ -2533,9 +2512,8 @@ extern "C" int dns2d_batch_get_scalars(dns2d_batch *b, int member, dns2d_scalars
 // device; forward / backward / training driven from here.
 // ============================================================================================
 // Autotuner: times the kernel variants of one size on a scratch state (k^4 field) and keeps
-// the fastest per (device, N).  The variants differ in rows per CTA (small grids), thread groups
-// per column CTA and L2 prefetch distances (large grids) and compute the same arithmetic, so a
-// tuned run gives the same results as an untuned one.  States and batches created afterwards on
+// the fastest per (device, N).  The variants of N <= 512 differ in rows per CTA (same arithmetic) and
+// radix plan (another rounding); the larger sizes have one configuration each.  States and batches created afterwards on
 // that device use the choice; DNS2D_AUTOTUNE=1 in the environment tunes at dns2d_create.
 // ============================================================================================
 namespace {
@@ -2579,7 +2557,7 @@ extern "C" int dns2d_autotune(int N, int device, int *config)
     const KernelSet *ks = kernel_set(N);
     if (!ks) return DNS2D_ERR_SIZE;
     Tuning best;
-    if (!cluster_size(N)) {  // the cluster sizes have a single configuration
+    if (!single_config(N)) {
         t_in_autotune = true;
         dns2d_state *s = nullptr;
         int rc = dns2d_create(&s, N, 1.0e5f, 4.0f, 0.1f, device);
@@ -2592,35 +2570,12 @@ extern "C" int dns2d_autotune(int N, int device, int *config)
             dns2d_destroy(s);
             return rc;
         }
-        const int reps = N >= 2048 ? 20 : 100;
-        const bool large = N >= 1024;
-        float tb = 1e30f;
-        if (large) {
-            for (int pf : {0, 148, 296, 444, 592}) {
-                s->tune = best;
-                s->tune.pf_rows = pf;
-                const Pointers p = s->ptrs();
-                const float t = time_launches(s, reps, [&] { ks->rows_step(p, s->stream, 1); });
-                if (t < tb) tb = t, best.pf_rows = pf;
-            }
-            tb = 1e30f;
-            for (int g : {1, 2})
-                for (int pf : {0, 37, 74, 148}) {
-                    s->tune = best;
-                    s->tune.cols_groups = g;
-                    s->tune.pf_cols = pf;
-                    const Pointers p = s->ptrs();
-                    const float t = time_launches(s, reps, [&] { ks->cols_step(p, 0, 0, s->stream, 1); });
-                    if (t < tb) tb = t, best.cols_groups = g, best.pf_cols = pf;
-                }
-        } else {
-            best = tune_small(ks->nplans, best, [&](const Tuning &t, bool rows) {
-                s->tune = t;
-                const Pointers p = s->ptrs();
-                if (rows) return time_launches(s, reps, [&] { ks->rows_step(p, s->stream, 1); });
-                return time_launches(s, reps, [&] { ks->cols_step(p, 0, 0, s->stream, 1); });
-            });
-        }
+        best = tune_small(ks->nplans, best, [&](const Tuning &t, bool rows) {
+            s->tune = t;
+            const Pointers p = s->ptrs();
+            if (rows) return time_launches(s, 100, [&] { ks->rows_step(p, s->stream, 1); });
+            return time_launches(s, 100, [&] { ks->cols_step(p, 0, 0, s->stream, 1); });
+        });
         const cudaError_t e = cudaStreamSynchronize(s->stream);
         dns2d_destroy(s);
         if (e != cudaSuccess) return DNS2D_ERR_CUDA;

@@ -5,19 +5,19 @@
 //               The reference keeps [iz][ix] (cuda/cuda_dns.h:62-63); the column pass reads
 //               whole kx columns, so the state is stored transposed here and converted at the
 //               API boundary.
-//   work      : [2][L/4][H][4] complex64.  Component c, physical row z, mode kx sits at
-//               ((z/4)*H + kx)*4 + z%4.  Between the column pass and the row pass it holds the
+//   work      : [L/4][H][4][2] complex64.  Component c, physical row z, mode kx sits at
+//               (((z/4)*H + kx)*4 + z%4)*2 + c: the 4 rows' two components of a mode are 64
+//               contiguous bytes.  Between the column pass and the row pass it holds the
 //               velocity after the z-inverse transform, U(z,kx) and W(z,kx); between the row
 //               pass and the column pass it holds the x-forward transforms of the products,
-//               D(z,kx) = F_x[u^2 - w^2] and E(z,kx) = F_x[u w].  Groups of 4 rows are
-//               contiguous per kx, so the row pass reads/writes whole 4-row tiles and the column
-//               pass moves full 32-byte sectors.
+//               D(z,kx) = F_x[u^2 - w^2] and E(z,kx) = F_x[u w].  A row pass of two rows moves
+//               whole 32-byte sectors, a column pass 64 contiguous bytes per 4 rows.
 //
 // One time step of the reference (cuda/mem_cuda.cu:1848-1857: STEP2B -> STEP3 -> STEP2A)
 // becomes two kernels:
-//   row pass    (k_rows_step):  U,W rows -> C2R -> u,w -> (u+iw)^2 -> R2C -> D,E rows
+//   row pass    (k_rows_step, large grids k_rows_ip):  U,W rows -> C2R -> u,w -> (u+iw)^2 -> R2C -> D,E rows
 //               = STEP2A's x-inverse + STEP2B's products and x-forward
-//   column pass (k_cols_step):  D,E columns -> z-forward (kz in [-N/2,N/2)) -> FN ->
+//   column pass (k_cols_step, large grids k_cols_ip):  D,E columns -> z-forward (kz in [-N/2,N/2)) -> FN ->
 //               Crank-Nicolson/AB2 update of om2, fnm1 <- FN -> velocity recovery ->
 //               3/2 zero-padding -> z-inverse -> U,W columns
 //               = STEP2B's z-forward + zero row N, STEP3, STEP2A's dealias/reshuffle/z-inverse
@@ -103,11 +103,21 @@ struct AltPlans<512> {
     using P2 = Radices<8, 8, 12>;
 };
 
-// work-buffer index (float2 units) of component c, physical row z, mode kx
+// work-buffer index (float2 units) of component c, physical row z, mode kx; consecutive kx of a row
+// are widx_kx_stride float2 apart
+constexpr int widx_rows = 4, widx_kx_stride = 2 * widx_rows;
 template <int L, int H>
 __device__ __forceinline__ size_t widx(int c, int z, int kx)
 {
-    return (size_t)c * ((size_t)L * H) + (((size_t)(z >> 2) * H + kx) << 2) + (z & 3);
+    return ((size_t)(z / widx_rows) * H + kx) * widx_kx_stride + ((z % widx_rows) << 1) + c;
+}
+
+// the same for a buffer of one component (the scalar diagnostics' scratch)
+constexpr int sidx_kx_stride = 4;
+template <int L, int H>
+__device__ __forceinline__ size_t widx1(int z, int kx)
+{
+    return ((size_t)(z >> 2) * H + kx) * sidx_kx_stride + (z & 3);
 }
 
 // parameters that change between segments of the run (read from device memory so a captured
@@ -135,10 +145,8 @@ struct Pointers {
     size_t s_state, s_work;
     int s_part, s_hist;
     // kernel configuration (the autotuner's choice; every choice gives the same arithmetic):
-    // rows per CTA of the small-grid row pass (0: the size's default), thread groups per column
-    // CTA of the large-grid column pass (0: default), L2 prefetch distances in CTAs (0: off)
-    int rows_tile = 0, cols_groups = 0;
-    int pf_rows = 296, pf_cols = 74;
+    // rows per CTA of the small-grid row pass (0: the size's default)
+    int rows_tile = 0;
     // radix plan of the small-grid row / column pass (0: Cfg<N>::Plan, 1, 2: AltPlans<N>); unlike
     // the knobs above a plan changes the FP32 rounding
     int plan_rows = 0, plan_cols = 0;
@@ -431,38 +439,69 @@ __global__ void __launch_bounds__(Cfg<N>::NTA) k_cols_step(Pointers p0, int firs
 }
 
 // ------------------------------------------------------------------------------------------
-// Large-grid variants: one row / one column per CTA, one butterfly per thread and stage, three
-// stages.  Row pass: inverse plan (R1, R2, R3), forward plan (R3, R2, R1) so that the inverse's
-// last stage leaves in registers exactly the stride-L/R3 elements the forward's first stage
-// needs: C2R -> products -> R2C runs through shared memory only four times.  The first inverse
-// stage reads U, W straight from global memory.  Column pass: plan (R3, R2, R1) both ways, the
-// forward's first stage read from global, the inverse's last stage written to global.
+// Large-grid transforms of the diagnostics: one row / one column per CTA, one butterfly per thread
+// and stage, three auto-sort stages.  The inverse's last stage leaves its outputs in registers, the
+// first one reads its inputs straight from global memory where they lie there.
 // ------------------------------------------------------------------------------------------
 template <int N_>
 struct Cfg2 {
     static constexpr bool enabled = false;
 };
 
-#define DNS2D_CFG2(N_, NT_, R1_, R2_, R3_, MC2_, MC4_, PS_)                                    \
+#define DNS2D_CFG2(N_, NT_, R1_, R2_, R3_, PS_)                                                \
     template <>                                                                                \
     struct Cfg2<N_> {                                                                          \
         static constexpr bool enabled = true;                                                  \
         static constexpr int PS = PS_; /* shared-memory padding: one float2 every 2^PS */       \
         static constexpr int N = N_, H = N_ / 2, L = 3 * N_ / 2, LP = SmemLen<L, PS_>::value;  \
         static constexpr int NT = NT_, R1 = R1_, R2 = R2_, R3 = R3_;                           \
-        static constexpr int MC2 = MC2_, MC4 = MC4_; /* CTAs per SM: k_cols_step2, k_cols_step4 */ \
         static_assert(R1_ * R2_ * R3_ == L, "plan");                                           \
         static_assert(L / R1_ <= NT_ && L / R2_ <= NT_ && L / R3_ <= NT_, "one butterfly");    \
     };
 // N = 4096 / 2048: plans (16, 24, 16) / (16, 12, 16) with padding every 16 elements make every
-// shared-memory access of both passes bank-conflict free (the radix-24 stage has Ns = 16, so its stores are contiguous per
-// half-warp, and the stride-16 stores of the Ns = 1 stages spread over all banks); the radix-16
-// middle stage of the row pass also holds 16 values in registers instead of 24.
-//          N    NT  plan (R1, R2, R3)  column CTAs per SM asked of the register allocator, pad
-DNS2D_CFG2(1024, 192, 16, 12, 8,       2, 1, 4)
-DNS2D_CFG2(2048, 256, 16, 12, 16,      2, 2, 4)  // two-group columns at 64 registers, 2 CTAs per SM
-DNS2D_CFG2(4096, 384, 16, 24, 16,      2, 1, 4)
+// shared-memory access bank-conflict free (the radix-24 stage has Ns = 16, so its stores are
+// contiguous per half-warp, and the stride-16 stores of the Ns = 1 stages spread over all banks).
+//          N    NT  plan (R1, R2, R3)  pad
+DNS2D_CFG2(1024, 192, 16, 12, 8,  4)
+DNS2D_CFG2(2048, 256, 16, 12, 16, 4)
+DNS2D_CFG2(4096, 384, 16, 24, 16, 4)
 #undef DNS2D_CFG2
+
+// Radix plan of an in-place transform (inplace.cuh); its forward half has the twiddle stages of the
+// auto-sort plan (R3, R2, R1).
+template <int L_, int R1_, int R2_, int R3_>
+struct InPlan {
+    static constexpr int L = L_, R1 = R1_, R2 = R2_, R3 = R3_, B1 = R2_ * R3_;
+    static_assert(R1_ * R2_ * R3_ == L_, "plan");
+    static_assert(R3_ % 8 == 0 && B1 % 32 == 0, "swizzle groups of 8, whole warps in the R1 stage");
+    using Tw = Radices<R3_, R2_, R1_>;
+};
+
+template <int N_>
+struct CfgI {
+    static constexpr bool enabled = false;
+};
+
+#define DNS2D_CFGI(N_, NTR_, MBR_, A1_, A2_, A3_, NTC_, MBC_, B1_, B2_, B3_)                   \
+    template <>                                                                                \
+    struct CfgI<N_> {                                                                          \
+        static constexpr bool enabled = true;                                                  \
+        static constexpr int N = N_, H = N_ / 2, L = 3 * N_ / 2;                               \
+        static constexpr int NTR = NTR_, MBR = MBR_, NTC = NTC_, MBC = MBC_;                   \
+        using RowPlan = InPlan<L, A1_, A2_, A3_>;                                              \
+        using ColPlan = InPlan<L, B1_, B2_, B3_>;                                              \
+    };
+// Threads per CTA, CTAs per SM asked of the register allocator and plan (R1, R2, R3), rows then
+// columns.  Shared memory (16 L bytes) allows 2 / 4 / 8 CTAs per SM at N = 4096 / 2048 / 1024; the
+// thread counts divide a stage's L / R butterflies into whole rounds where they can.  Other
+// choices measured on B200 (rows, columns in us): 4096 rows 256 threads 201, columns 128 threads 217,
+// 256 threads 217, plan (24, 32, 8) 226; 2048 rows 64 threads 55.5, columns (16, 12, 16) 55, rows
+// (16, 24, 8) 54.5; 1024 (few CTAs per SM: more threads each) 64 threads 21.6 / 25.8.
+//          N     rows: NT MB  plan        columns: NT MB  plan
+DNS2D_CFGI(1024,      128, 4, 16, 12, 8,           128, 4, 16, 12, 8)
+DNS2D_CFGI(2048,      128, 4, 16, 12, 16,          128, 4, 16, 24, 8)
+DNS2D_CFGI(4096,      128, 2, 16, 24, 16,          192, 2, 16, 24, 16)
+#undef DNS2D_CFGI
 
 // twiddle catalog of size N: the stages of every plan compiled for it
 template <int N>
@@ -478,6 +517,10 @@ constexpr TwCatalog make_catalog()
         c.add(Radices<Cfg2<N>::R1, Cfg2<N>::R2, Cfg2<N>::R3>{});
         c.add(Radices<Cfg2<N>::R3, Cfg2<N>::R2, Cfg2<N>::R1>{});
     }
+    if constexpr (CfgI<N>::enabled) {
+        c.add(typename CfgI<N>::RowPlan::Tw{});
+        c.add(typename CfgI<N>::ColPlan::Tw{});
+    }
     return c;
 }
 
@@ -488,12 +531,12 @@ struct TwCat {
 };
 
 // Inverse x transform of a row pair on the large-grid plan: the half spectra A = U[k], B = W[k]
-// (k < H, consecutive k 4 float2 apart, as in the work layout) of two real rows a, b are packed
+// (k < H, consecutive k KS float2 apart) of two real rows a, b are packed
 // Hermitian-wise as A + iB and transformed (C2R semantics: only Re of the k = 0 entries is used).
 // Thread j < L/R3 is left holding v[q] = (a(x), b(x)) at x = j + q L/R3; the last inverse stage
-// runs in registers.  Used by the row pass (rows u, w of one physical row), NEXTDT (the same,
-// for the CFL maximum) and OM2PHYS (two physical rows of one field).
-template <int N>
+// runs in registers.  Used by NEXTDT (rows u, w of one physical row, for the CFL maximum) and
+// OM2PHYS (two physical rows of one field).
+template <int N, int KS>
 __device__ __forceinline__ void rows_inverse2(const float2 *__restrict__ U, const float2 *__restrict__ W, float2 *s,
                                               const float2 *__restrict__ tw, float2 (&v)[Cfg2<N>::R3])
 {
@@ -518,8 +561,8 @@ __device__ __forceinline__ void rows_inverse2(const float2 *__restrict__ U, cons
             b[r] = a[r];
             const int k = jb + r * LR1;
             if (!slot_in_band<L, R1, H, L - H>(r) && r * LR1 < H && k < H) {
-                a[r] = U[(size_t)k << 2];
-                b[r] = W[(size_t)k << 2];
+                a[r] = U[(size_t)k * KS];
+                b[r] = W[(size_t)k * KS];
             }
         }
         float2 v[R1];
@@ -565,185 +608,6 @@ __device__ __forceinline__ void rows_inverse2(const float2 *__restrict__ U, cons
     }
 }
 
-// three CTAs per SM: the register allocator keeps the row pass at 56 registers (36 warps per SM;
-// N = 4096: 0.311 -> 0.280 ms against two CTAs at 80 registers)
-template <int N>
-__global__ void __launch_bounds__(Cfg2<N>::NT, 3) k_rows_step2(Pointers p0)
-{
-    const Pointers p = p0.member(blockIdx.y);
-    using C = Cfg2<N>;
-    constexpr int L = C::L, H = C::H, R1 = C::R1, R2 = C::R2, R3 = C::R3, PS = C::PS;
-    constexpr int LR3 = L / R3;
-    extern __shared__ float2 s[];
-    const int z = blockIdx.x;
-    const int j = threadIdx.x;
-    const float2 *__restrict__ U = p.work + widx<L, H>(0, z, 0);
-    const float2 *__restrict__ W = p.work + widx<L, H>(1, z, 0);
-    // bring to L2 the quarter (z % 4) of the 4-row tile that the CTA pf_rows later reads (two
-    // waves of 148 SMs x 2 CTAs by default)
-    if (p.pf_rows > 0 && z + p.pf_rows < L) {
-        const int t = (z + p.pf_rows) >> 2, part = z & 3;
-        constexpr int QB = H * 32 / 4;  // bytes of one quarter tile of one component
-        const char *b0 = reinterpret_cast<const char *>(p.work + (size_t)t * H * 4) + part * QB;
-        for (int o = j * 128; o < 2 * QB; o += C::NT * 128)
-            prefetch_l2(o < QB ? b0 + o : b0 + (size_t)L * H * 8 + (o - QB));
-    }
-    // inverse x transform; its last stage leaves u + i w in registers -> products -> forward
-    // stage 1
-    float2 v[R3];
-    rows_inverse2<N>(U, W, s, p.tw, v);
-    if (j < LR3) {
-#pragma unroll
-        for (int q = 0; q < R3; ++q) v[q] = make_float2(v[q].x * v[q].x - v[q].y * v[q].y, 2.0f * v[q].x * v[q].y);
-        DFT<R3, false>::run(v);
-    }
-    __syncthreads();
-    if (j < LR3) sm_store<L, R3, 1, PS>(s, v, j);
-    stage1<TwCat<N>, L, R2, R3, false, PS>(s, p.tw);
-    // the unpack reads Q[k] and Q[L-k] for k < H: positions in [H, L-H] are never read
-    stage1_last_band<TwCat<N>, L, R1, false, H, L - H, PS>(s, p.tw);
-    __syncthreads();
-    float2 *__restrict__ Do = p.work + widx<L, H>(0, z, 0);
-    float2 *__restrict__ Eo = p.work + widx<L, H>(1, z, 0);
-    for (int k = j; k < H; k += C::NT) {
-        const float2 q = s[sidx<PS>(k)];
-        const float2 m = s[sidx<PS>(k == 0 ? 0 : L - k)];
-        Do[(size_t)k << 2] = make_float2(0.5f * (q.x + m.x), 0.5f * (q.y - m.y));
-        Eo[(size_t)k << 2] = make_float2(0.25f * (q.y + m.y), -0.25f * (q.x - m.x));
-    }
-}
-
-template <int N>
-__global__ void __launch_bounds__(Cfg2<N>::NT, Cfg2<N>::MC2) k_cols_step2(Pointers p0, int first, int hist_slot)
-{
-    const Pointers p = p0.member(blockIdx.y);
-    using C = Cfg2<N>;
-    constexpr int L = C::L, H = C::H, LP = C::LP, NT = C::NT, R1 = C::R1, R2 = C::R2, R3 = C::R3, PS = C::PS;
-    constexpr int LR1 = L / R1, LR3 = L / R3;
-    extern __shared__ float2 smem[];
-    __shared__ double2 red[32];
-    __shared__ bool am_last;
-    const int kx = blockIdx.x;
-    const int j = threadIdx.x;
-    float2 *sD = smem, *sE = smem + LP;
-    float2 *om2c = p.om2 + (size_t)kx * N;
-    float2 *fnc = p.fnm1 + (size_t)kx * N;
-    // the state column is only needed after the forward transforms: start bringing it to L2
-    for (int o = j * 32; o < N; o += NT * 32) {
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(om2c + o));
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(fnc + o));
-    }
-    // forward transforms of D and E along z, plan (R3, R2, R1): the twiddle-free radix-R3 first
-    // stage reads straight from global memory
-#pragma unroll 1
-    for (int a = 0; a < 2; ++a) {
-        float2 *s = a ? sE : sD;
-        if (j < LR3) {
-            // element j + r L/R3 of the column; L/R3 is a multiple of 4, so consecutive r are a
-            // fixed stride apart (one live address instead of R3)
-            static_assert(LR3 % 4 == 0, "stride");
-            constexpr size_t RS = (size_t)(LR3 / 4) * H * 4;
-            const float2 *ptr = p.work + widx<L, H>(a, j, kx);
-            float2 v[R3];
-#pragma unroll
-            for (int r = 0; r < R3; ++r, ptr += RS) v[r] = *ptr;
-            DFT<R3, false>::run(v);
-            sm_store<L, R3, 1, PS>(s, v, j);
-        }
-        stage1<TwCat<N>, L, R2, R3, false, PS>(s, p.tw);
-        stage1<TwCat<N>, L, R1, R3 * R2, false, PS>(s, p.tw);
-    }
-    __syncthreads();
-
-    const StepParams prm = *p.prm;
-    const float dt = prm.dt;
-    const float cnm1 = first ? prm.cnm1_first : prm.cn;
-    const double hvdt = 0.5 * (double)prm.visc * (double)dt;
-    const double c2n = 0.5 * (double)dt * (2.0 + (double)cnm1);
-    const double c3n = -0.5 * (double)dt * (double)cnm1;
-    const float divxz = (float)(1.0 / ((double)L * (double)L));
-    double2 ez = make_double2(0.0, 0.0);
-    const double wgt = (kx == 0) ? 0.5 : 1.0;
-    for (int iz = j; iz < N; iz += NT) {
-        const int kz = (iz < H) ? iz : iz - N;
-        const int kzi = (kz >= 0) ? kz : kz + L;
-        const float2 d = sD[sidx<PS>(kzi)];
-        const float2 e = sE[sidx<PS>(kzi)];
-        float2 fn = make_float2(0.f, 0.f);
-        if (kz != -H) {
-            const float ga = (float)kz * (float)kx;
-            const float g2a2 = (float)kz * (float)kz - (float)kx * (float)kx;
-            fn.x = (ga * d.x + g2a2 * e.x) * divxz;
-            fn.y = (ga * d.y + g2a2 * e.y) * divxz;
-            if (p.force) fn = add_forcing(fn, p, kx, iz, N);
-        }
-        const double K2 = (double)kx * kx + (double)kz * kz;
-        const float2 on = cn_update(om2c[iz], fn, fnc[iz], K2, hvdt, c2n, c3n);
-        om2c[iz] = on;
-        fnc[iz] = fn;
-        float2 u, w;
-        double invK2;
-        recover_velocity(kx, kz, on, u, w, invK2);
-        sD[sidx<PS>(kzi)] = u;
-        sE[sidx<PS>(kzi)] = w;
-        const double pw = (double)on.x * on.x + (double)on.y * on.y;
-        ez.x += wgt * pw * invK2;
-        ez.y += wgt * pw;
-    }
-    for (int z = H + j; z < L - H; z += NT) {
-        sD[sidx<PS>(z)] = make_float2(0.f, 0.f);
-        sE[sidx<PS>(z)] = make_float2(0.f, 0.f);
-    }
-    ez = block_sum2<NT>(ez, red);
-    if (threadIdx.x == 0) {
-        p.part[kx] = ez;
-        __threadfence();
-        const unsigned int n = atomicAdd(p.counter, 1u);
-        am_last = (n == gridDim.x - 1);
-    }
-    __syncthreads();
-    if (am_last) {
-        double2 acc = make_double2(0.0, 0.0);
-        for (int i = threadIdx.x; i < H; i += NT) {
-            const double2 q = __ldcg(&p.part[i]);
-            acc.x += q.x;
-            acc.y += q.y;
-        }
-        acc = block_sum2<NT>(acc, red);
-        if (threadIdx.x == 0) {
-            p.hist[hist_slot] = acc;
-            *p.counter = 0u;
-        }
-    }
-    // inverse transforms along z, plan (R3, R2, R1), the last stage straight to global memory
-#pragma unroll 1
-    for (int a = 0; a < 2; ++a) {
-        float2 *s = a ? sE : sD;
-        stage1<TwCat<N>, L, R3, 1, true, PS>(s, p.tw);
-        stage1<TwCat<N>, L, R2, R3, true, PS>(s, p.tw);
-        __syncthreads();
-        if (j < LR1) {
-            float2 v[R1];
-            sm_load<L, R1, PS>(v, s, j);
-            bfly<TwCat<N>, L, R1, LR1, true>(v, j, p.tw);
-            static_assert(LR1 % 4 == 0, "stride");
-            constexpr size_t QS = (size_t)(LR1 / 4) * H * 4;
-            float2 *ptr = p.work + widx<L, H>(a, j, kx);
-#pragma unroll
-            for (int q = 0; q < R1; ++q, ptr += QS) *ptr = v[q];
-        }
-    }
-}
-
-// ------------------------------------------------------------------------------------------
-// Column pass with one CTA of two thread groups per column: group 0 transforms D (then U),
-// group 1 E (then W), each group synchronising on its own named barrier; the spectral update
-// uses the whole CTA.  Same arithmetic as k_cols_step2.  One 768-thread CTA per SM holds half
-// the shared memory of two 384-thread CTAs with the same number of warps, which leaves L1 room
-// for the twiddle tables (N = 4096 on B200: 0.680 -> 0.655 ms per step; no register spills at
-// 80 registers, where the single-group kernel spilled 272 bytes).  The columns arrive by
-// cp.async (no registers held by loads in flight) and the state column is prefetched to L2.
-// ------------------------------------------------------------------------------------------
 template <int NTH>
 __device__ __forceinline__ void group_sync(int id)
 {
@@ -782,176 +646,6 @@ __device__ __forceinline__ void stage1g_first_band(float2 *s, const float2 *tw, 
     if (j < LR) sm_store<L, R, 1, PS>(s, v, j);
 }
 
-template <class Cat, int L, int R, bool INV, int NTH, int B0, int B1, int PS = 5>
-__device__ __forceinline__ void stage1g_last_band(float2 *s, const float2 *tw, int j, int bar)
-{
-    constexpr int LR = L / R;
-    float2 v[R];
-    group_sync<NTH>(bar);
-    if (j < LR) {
-        sm_load<L, R, PS>(v, s, j);
-        bfly<Cat, L, R, LR, INV>(v, j, tw);
-    }
-    group_sync<NTH>(bar);
-    if (j < LR) {
-#pragma unroll
-        for (int q = 0; q < R; ++q)
-            if (!slot_in_band<L, R, B0, B1>(q)) s[sidx<PS>(j + q * LR)] = v[q];
-    }
-}
-
-// Where one column CTA holds an SM (MC4 = 1), the column's om2 / fnm1 are brought into shared
-// memory by cp.async at the start of the column pass, behind the D, E columns, so the spectral
-// update reads them with no global-load latency left (N = 4096 on B200: column pass 0.299 ->
-// 0.294 ms).  With two CTAs per SM the 2 x 16 N bytes more shrink L1 below the twiddle tables
-// (N = 2048: 0.075 -> 0.076 ms), so there the state is read from global memory, prefetched to L2.
-template <int N>
-constexpr bool cols4_stage_state()
-{
-    return Cfg2<N>::MC4 == 1;
-}
-
-// dynamic shared memory of k_cols_step4: the D / E (then U / W) arrays and the staged state
-template <int N>
-constexpr size_t cols4_smem_bytes()
-{
-    return (2 * (size_t)Cfg2<N>::LP + (cols4_stage_state<N>() ? 2 * (size_t)N : 0)) * sizeof(float2);
-}
-
-template <int N>
-__global__ void __launch_bounds__(2 * Cfg2<N>::NT, Cfg2<N>::MC4) k_cols_step4(Pointers p0, int first, int hist_slot)
-{
-    const Pointers p = p0.member(blockIdx.y);
-    using C = Cfg2<N>;
-    constexpr int L = C::L, H = C::H, LP = C::LP, NT = C::NT, NT2 = 2 * C::NT, PS = C::PS;
-    constexpr int R1 = C::R1, R2 = C::R2, R3 = C::R3, LR1 = L / R1;
-    static_assert(NT % 32 == 0, "groups must be whole warps");
-    extern __shared__ float2 smem[];
-    __shared__ double2 red[32];
-    __shared__ bool am_last;
-    const int kx = blockIdx.x;
-    const int g = (int)threadIdx.x / NT;  // 0: D / U, 1: E / W
-    const int j = (int)threadIdx.x - g * NT;
-    const int bar = 1 + g;
-    float2 *sD = smem, *sE = smem + LP;
-    float2 *sg = smem + g * LP;
-    float2 *om2c = p.om2 + (size_t)kx * N;
-    float2 *fnc = p.fnm1 + (size_t)kx * N;
-    for (int z = j; z < L; z += NT) cp_async8(sg + sidx<PS>(z), p.work + widx<L, H>(g, z, kx));
-    cp_async_commit();
-    constexpr bool STAGE = cols4_stage_state<N>();
-    float2 *so = smem + 2 * LP, *sf = so + N;  // the staged state column, dense (read at consecutive iz)
-    if constexpr (STAGE) {
-        for (int i = (int)threadIdx.x; i < N; i += NT2) {
-            cp_async8(so + i, om2c + i);
-            cp_async8(sf + i, fnc + i);
-        }
-        cp_async_commit();
-    } else {
-        for (int o = (int)threadIdx.x * 16; o < N; o += NT2 * 16) {
-            prefetch_l2(om2c + o);
-            prefetch_l2(fnc + o);
-        }
-    }
-    if (p.pf_cols > 0 && kx + p.pf_cols < (int)gridDim.x) {  // the column pf_cols CTAs later
-        const int kp = kx + p.pf_cols;
-        for (int q = (int)threadIdx.x; q < 2 * (L / 4); q += NT2) {
-            const int a = q / (L / 4), gg = q - a * (L / 4);
-            prefetch_l2(p.work + (size_t)a * L * H + (((size_t)gg * H + kp) << 2));
-        }
-    }
-    cp_async_wait<STAGE ? 1 : 0>();  // this thread's D / E copies have landed
-    stage1g<TwCat<N>, L, R3, 1, false, NT, PS>(sg, p.tw, j, bar);
-    stage1g<TwCat<N>, L, R2, R3, false, NT, PS>(sg, p.tw, j, bar);
-    // the update reads kz_i < H and kz_i >= L - H only: the 3/2 band [H, L-H-1] is not stored
-    stage1g_last_band<TwCat<N>, L, R1, false, NT, H, L - H - 1, PS>(sg, p.tw, j, bar);
-    cp_async_wait<0>();  // and the state copies
-    __syncthreads();
-
-    const StepParams prm = *p.prm;
-    const float dt = prm.dt;
-    const float cnm1 = first ? prm.cnm1_first : prm.cn;
-    const double hvdt = 0.5 * (double)prm.visc * (double)dt;
-    const double c2n = 0.5 * (double)dt * (2.0 + (double)cnm1);
-    const double c3n = -0.5 * (double)dt * (double)cnm1;
-    const float divxz = (float)(1.0 / ((double)L * (double)L));
-    double2 ez = make_double2(0.0, 0.0);
-    const double wgt = (kx == 0) ? 0.5 : 1.0;
-    for (int iz = (int)threadIdx.x; iz < N; iz += NT2) {
-        const int kz = (iz < H) ? iz : iz - N;
-        const int kzi = (kz >= 0) ? kz : kz + L;
-        const float2 d = sD[sidx<PS>(kzi)];
-        const float2 e = sE[sidx<PS>(kzi)];
-        float2 fn = make_float2(0.f, 0.f);
-        if (kz != -H) {
-            const float ga = (float)kz * (float)kx;
-            const float g2a2 = (float)kz * (float)kz - (float)kx * (float)kx;
-            fn.x = (ga * d.x + g2a2 * e.x) * divxz;
-            fn.y = (ga * d.y + g2a2 * e.y) * divxz;
-            if (p.force) fn = add_forcing(fn, p, kx, iz, N);
-        }
-        const double K2 = (double)kx * kx + (double)kz * kz;
-        const float2 on = STAGE ? cn_update(so[iz], fn, sf[iz], K2, hvdt, c2n, c3n)
-                                : cn_update(om2c[iz], fn, fnc[iz], K2, hvdt, c2n, c3n);
-        om2c[iz] = on;
-        fnc[iz] = fn;
-        float2 u, w;
-        double invK2;
-        recover_velocity(kx, kz, on, u, w, invK2);
-        sD[sidx<PS>(kzi)] = u;
-        sE[sidx<PS>(kzi)] = w;
-        const double pw = (double)on.x * on.x + (double)on.y * on.y;
-        ez.x += wgt * pw * invK2;
-        ez.y += wgt * pw;
-    }
-    ez = block_sum2<NT2>(ez, red);
-    if (threadIdx.x == 0) {
-        p.part[kx] = ez;
-        __threadfence();
-        const unsigned int n = atomicAdd(p.counter, 1u);
-        am_last = (n == gridDim.x - 1);
-    }
-    __syncthreads();
-    if (am_last) {
-        double2 acc = make_double2(0.0, 0.0);
-        for (int i = (int)threadIdx.x; i < H; i += NT2) {
-            const double2 q = __ldcg(&p.part[i]);
-            acc.x += q.x;
-            acc.y += q.y;
-        }
-        acc = block_sum2<NT2>(acc, red);
-        if (threadIdx.x == 0) {
-            p.hist[hist_slot] = acc;
-            *p.counter = 0u;
-        }
-    }
-    // 3/2 zero padding: the band [H, L-H-1] enters the first inverse stage as compile-time zeros
-    // where whole radix-R3 slots lie in it; band positions in a slot that also holds retained
-    // modes are read from shared memory, so they are cleared here (none when the slots tile the
-    // band exactly, as with R3 = 12 or 24)
-    for (int z = H + (int)threadIdx.x; z < L - H; z += NT2) {
-        if (!slot_in_band<L, R3, H, L - H - 1>(z / (L / R3))) {
-            sD[sidx<PS>(z)] = make_float2(0.f, 0.f);
-            sE[sidx<PS>(z)] = make_float2(0.f, 0.f);
-        }
-    }
-    __syncthreads();
-    // inverse transform of this group's column, plan (R3, R2, R1), last stage straight to HBM
-    stage1g_first_band<TwCat<N>, L, R3, true, NT, H, L - H - 1, PS>(sg, p.tw, j, bar);
-    stage1g<TwCat<N>, L, R2, R3, true, NT, PS>(sg, p.tw, j, bar);
-    group_sync<NT>(bar);
-    if (j < LR1) {
-        float2 v[R1];
-        sm_load<L, R1, PS>(v, sg, j);
-        bfly<TwCat<N>, L, R1, LR1, true>(v, j, p.tw);
-        static_assert(LR1 % 4 == 0, "stride");
-        constexpr size_t QS = (size_t)(LR1 / 4) * H * 4;
-        float2 *ptr = p.work + widx<L, H>(g, j, kx);
-#pragma unroll
-        for (int q = 0; q < R1; ++q, ptr += QS) *ptr = v[q];
-    }
-}
-
 // ------------------------------------------------------------------------------------------
 // Diagnostics on the large-grid plans (the sizes with Cfg2): NEXTDT's CFL maximum and the
 // physical velocity planes (as k_rows_velocity), and OM2PHYS / the stream function (as
@@ -969,7 +663,7 @@ __global__ void __launch_bounds__(Cfg2<N>::NT, 3) k_rows_velocity2(Pointers p0, 
     __shared__ float red[32];
     const int z = blockIdx.x, j = threadIdx.x;
     float2 v[R3];
-    rows_inverse2<N>(p.work + widx<L, H>(0, z, 0), p.work + widx<L, H>(1, z, 0), s, p.tw, v);
+    rows_inverse2<N, widx_kx_stride>(p.work + widx<L, H>(0, z, 0), p.work + widx<L, H>(1, z, 0), s, p.tw, v);
     float m = 0.0f;
     if (j < LR3) {
 #pragma unroll
@@ -1018,7 +712,7 @@ __global__ void __launch_bounds__(Cfg2<N>::NT) k_cols_scalar2(Pointers p, float2
         sm_load<L, R1, PS>(v, s, j);
         bfly<TwCat<N>, L, R1, LR1, true>(v, j, p.tw);
         constexpr size_t QS = (size_t)(LR1 / 4) * H * 4;
-        float2 *ptr = scratch + widx<L, H>(0, j, kx);
+        float2 *ptr = scratch + widx1<L, H>(j, kx);
 #pragma unroll
         for (int q = 0; q < R1; ++q, ptr += QS) *ptr = v[q];
     }
@@ -1036,7 +730,7 @@ __global__ void __launch_bounds__(Cfg2<N>::NT, 3) k_rows_pair2(Pointers p, const
     __shared__ float red[32];
     const int z = 2 * blockIdx.x, j = threadIdx.x;
     float2 v[R3];
-    rows_inverse2<N>(scratch + widx<L, H>(0, z, 0), scratch + widx<L, H>(0, z + 1, 0), s, p.tw, v);
+    rows_inverse2<N, sidx_kx_stride>(scratch + widx1<L, H>(z, 0), scratch + widx1<L, H>(z + 1, 0), s, p.tw, v);
     float mn = 3.402823466e38f, mx = -3.402823466e38f;
     if (j < LR3) {
 #pragma unroll
@@ -1194,7 +888,7 @@ __global__ void __launch_bounds__(Cfg<N>::NTA) k_cols_scalar(Pointers p, float2 
     for (int z = H + threadIdx.x; z < L - H; z += NT) smem[sidx<PS>(z)] = make_float2(0.f, 0.f);
     __syncthreads();
     fft_run<TwCat<N>, L, LP, true, 1, NT, PS>(smem, p.tw, typename C::Plan{});
-    for (int z = threadIdx.x; z < L; z += NT) scratch[widx<L, H>(0, z, kx)] = smem[sidx<PS>(z)];
+    for (int z = threadIdx.x; z < L; z += NT) scratch[widx1<L, H>(z, kx)] = smem[sidx<PS>(z)];
 }
 
 // scratch rows -> real field rows written to out ([L][L]); per-block min/max partials
@@ -1210,7 +904,7 @@ __global__ void __launch_bounds__(Cfg<N>::NTB) k_rows_scalar(Pointers p, const f
     const int z0 = blockIdx.x * ROWS;
     for (int e = threadIdx.x; e < ROWS * H; e += NT) {
         const int r = e % ROWS, k = e / ROWS;
-        const float2 a = scratch[widx<L, H>(0, z0 + r, k)];
+        const float2 a = scratch[widx1<L, H>(z0 + r, k)];
         float2 *x = smem + r * LP;
         if (k == 0) {
             x[sidx<PS>(0)] = make_float2(a.x, 0.f);
@@ -1265,7 +959,7 @@ __global__ void __launch_bounds__(Cfg<N>::NTB) k_rows_fwd_scalar(Pointers p, con
     for (int e = threadIdx.x; e < ROWS * H; e += NT) {
         const int r = e % ROWS, k = e / ROWS;
         const float2 q = smem[r * LP + sidx<PS>(k)];
-        scratch[widx<L, H>(0, z0 + r, k)] = make_float2(q.x * sc, q.y * sc);
+        scratch[widx1<L, H>(z0 + r, k)] = make_float2(q.x * sc, q.y * sc);
     }
 }
 
@@ -1304,7 +998,7 @@ __global__ void __launch_bounds__(Cfg<N>::NTA) k_cols_fwd_scalar(Pointers p, con
     __shared__ double sp[NT], sz[NT];
     __shared__ bool last;
     const int kx = blockIdx.x;
-    for (int z = threadIdx.x; z < L; z += NT) smem[sidx<PS>(z)] = scratch[widx<L, H>(0, z, kx)];
+    for (int z = threadIdx.x; z < L; z += NT) smem[sidx<PS>(z)] = scratch[widx1<L, H>(z, kx)];
     __syncthreads();
     fft_run<TwCat<N>, L, LP, false, 1, NT, PS>(smem, p.tw, typename C::Plan{});
     const float sc = 1.0f / (float)L;

@@ -1,0 +1,455 @@
+// inplace.cuh — the step's row and column passes on in-place transforms (the sizes with CfgI).
+//
+// A CTA holds two sequences of length L = R1 R2 R3 side by side: two physical rows (row pass), or
+// the D and E (then U and W) columns of one kx (column pass).  An element is 16 bytes in shared
+// memory, (re, re', im, im'), so one 128-bit access moves both sequences' values and every butterfly
+// operation is one packed instruction on both (cpair, fft.cuh).
+//
+// Every stage is in place: a butterfly writes its outputs to the positions its inputs came from,
+// so nothing is held in registers across a barrier and one barrier separates two stages (the
+// auto-sort stages of fft.cuh need two, and the registers of all threads in between).  The first
+// transform of a pass runs natural -> digit-reversed order (decimation in frequency: radix R1 over
+// the L/R1-strided digit, then R2, then R3 over R3 contiguous elements), the second one
+// digit-reversed -> natural (decimation in time, R3, R2, R1), and what lies between the two (the
+// products of the row pass, the spectral update of the column pass) works in any order.  So no
+// reordering pass exists, and the R3 stages of both transforms with everything between them run in
+// registers: a pass touches shared memory 4 times in each direction.
+//   position p = i1 B1 + i2 R3 + i3 (B1 = R2 R3) holds
+//     row pass:     kx = p before, x = i1 + R1 (i2 + R2 i3) between, kx = p after
+//     column pass:  z = p before, kz = i1 + R1 (i2 + R2 i3) between, z = p after
+// In the row pass, between the two outer stages a warp works on its own blocks of B1 elements only
+// (no CTA barrier: two per pass in all).  Bank conflicts: i3 is stored as i3 ^ ((i1 ^ i2) & 7), so
+// eight neighbouring lanes find eight different 16-byte columns in every stage, along i3, i2 or i1.
+//
+// Bounds (N = 4096 on B200, 1965 MHz; ncu): the row pass is bound by the L1 / shared-memory data
+// pipe (67-75 % of its cycles busy; 24 % before the loads' and twiddles' share fell), the column pass
+// by the latency of its phases at two CTAs per SM (HBM 35 %, issue 32 %).  Measured (rows / columns,
+// one launch): N = 4096 0.254 / 0.293 -> 0.186 / 0.211 ms, N = 2048 67.6 / 71.7 -> 50.8 / 51.0 us,
+// N = 1024 27.0 / 28.2 -> 20.1 / 23.6 us against the auto-sort kernels that these replace (one row,
+// or one array and thread group, per 384 threads).
+// Tried and slower, or no faster: each sequence on its own lane with scalar butterflies (rows 0.185,
+// columns 0.223 ms at N = 4096), fetching the next round's twiddles, state or rows into registers
+// (columns 0.220-0.239 ms), prefetching a later CTA's input to L2 (columns +4 us), twice the threads at
+// half the registers (rows 0.200 ms), 2-row tiles of the work buffer (columns 0.259 ms).
+#pragma once
+#include "dns2d_kernels.cuh"
+
+namespace dns2d {
+
+// shared-memory element <-> the two complex values of a butterfly input
+__device__ __forceinline__ cpair ip_get(const float4 *s, int i)
+{
+    const float4 x = s[i];
+    return {make_float2(x.x, x.y), make_float2(x.z, x.w)};
+}
+__device__ __forceinline__ void ip_put(float4 *s, int i, cpair v)
+{
+    s[i] = make_float4(v.re.x, v.re.y, v.im.x, v.im.y);
+}
+// element r of a butterfly whose element 0 has the (swizzled) index b; the elements are STRIDE apart
+template <int R, int STRIDE>
+__device__ __forceinline__ void ip_load(cpair (&v)[R], const float4 *s, int b)
+{
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = ip_get(s, (b ^ (r & 7)) + r * STRIDE);
+}
+template <int R, int STRIDE>
+__device__ __forceinline__ void ip_store(float4 *s, const cpair (&v)[R], int b)
+{
+#pragma unroll
+    for (int r = 0; r < R; ++r) ip_put(s, (b ^ (r & 7)) + r * STRIDE, v[r]);
+}
+// the same for the R contiguous elements of a group
+template <int R>
+__device__ __forceinline__ void ip_load_run(cpair (&v)[R], const float4 *s, int b)
+{
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = ip_get(s, (b ^ (r & 7)) + (r & ~7));
+}
+template <int R>
+__device__ __forceinline__ void ip_store_run(float4 *s, const cpair (&v)[R], int b)
+{
+#pragma unroll
+    for (int r = 0; r < R; ++r) ip_put(s, (b ^ (r & 7)) + (r & ~7), v[r]);
+}
+
+// w[r] = W^{r k}, r >= 1: the twiddles of the stage (R, NS) at index k
+template <class Cat, int R, int NS>
+__device__ __forceinline__ void ip_tw_load(float2 (&w)[R], const float2 *__restrict__ tw, int k)
+{
+    constexpr int OFF = Cat::off(R, NS);
+    static_assert(OFF >= 0, "stage missing from the twiddle catalog");
+    const float2 *t = tw + OFF + k;
+#pragma unroll
+    for (int r = 1; r < R; ++r)
+        asm volatile("ld.global.nc.v2.f32 {%0, %1}, [%2];" : "=f"(w[r].x), "=f"(w[r].y) : "l"(t + (r - 1) * NS));
+}
+// v[r] *= w[r] (conjugate when INV)
+template <int R, bool INV>
+__device__ __forceinline__ void ip_twiddle(cpair (&v)[R], const float2 (&w)[R])
+{
+#pragma unroll
+    for (int r = 1; r < R; ++r) v[r] = cmul(v[r], INV ? cconj(w[r]) : w[r]);
+}
+
+// the two components of one mode on two neighbouring rows: 32 contiguous bytes of the work buffer
+struct row2 {
+    float4 a, b;
+};
+__device__ __forceinline__ row2 ld_row2(const float2 *p)
+{
+    row2 v;
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(v.a.x), "=f"(v.a.y), "=f"(v.a.z), "=f"(v.a.w), "=f"(v.b.x), "=f"(v.b.y), "=f"(v.b.z), "=f"(v.b.w)
+                 : "l"(p));
+    return v;
+}
+__device__ __forceinline__ void st_row2(float2 *p, const row2 &v)
+{
+    asm volatile("st.global.v8.f32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};" ::"f"(v.a.x), "f"(v.a.y), "f"(v.a.z),
+                 "f"(v.a.w), "f"(v.b.x), "f"(v.b.y), "f"(v.b.z), "f"(v.b.w), "l"(p)
+                 : "memory");
+}
+__device__ __forceinline__ cpair shfl_xor16(cpair m)
+{
+    cpair h;
+    h.re.x = __shfl_xor_sync(0xffffffffu, m.re.x, 16);
+    h.re.y = __shfl_xor_sync(0xffffffffu, m.re.y, 16);
+    h.im.x = __shfl_xor_sync(0xffffffffu, m.im.x, 16);
+    h.im.y = __shfl_xor_sync(0xffffffffu, m.im.y, 16);
+    return h;
+}
+
+// ------------------------------------------------------------------------------------------
+// Row pass: rows 2 blockIdx.x and + 1: U, W -> C2R -> (u + iw)^2 -> R2C -> D, E.
+// The Hermitian packing needs modes k and L - k together: k = j + r B1 is slot r of butterfly j, and
+// L - k is slot R1 - 1 - r of butterfly B1 - j, so butterflies j and B1 - j run 16 lanes apart in one
+// warp and exchange those slots by shuffle, on the way in and on the way out (butterflies 0 and
+// B1 / 2 are their own mirrors).
+// ------------------------------------------------------------------------------------------
+template <int N>
+__global__ void __launch_bounds__(CfgI<N>::NTR, CfgI<N>::MBR) k_rows_ip(Pointers p0)
+{
+    const Pointers p = p0.member(blockIdx.y);
+    using C = CfgI<N>;
+    using P = typename C::RowPlan;
+    using Cat = TwCat<N>;
+    constexpr int L = C::L, H = C::H, NT = C::NTR, R1 = P::R1, R2 = P::R2, R3 = P::R3, B1 = P::B1;
+    constexpr int NW = NT / 32, BPW = R1 / NW;  // blocks of B1 elements per warp
+    static_assert(R1 % NW == 0 && B1 % 32 == 0, "whole blocks per warp");
+    constexpr int NLO = (H + B1 - 1) / B1;  // slots with retained modes below H
+    extern __shared__ __align__(16) float4 s4[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    float2 *__restrict__ row = p.work + widx<L, H>(0, 2 * blockIdx.x, 0);
+    auto jof = [](int t) {  // butterfly of index t
+        const int l = t & 31, q = (t >> 5) * 16 + (l & 15);
+        return (l < 16) ? q : (q == 0 ? B1 / 2 : B1 - q);
+    };
+    float2 w1[R1], w2[R2];
+    ip_tw_load<Cat, R1, B1>(w1, p.tw, jof(tid < B1 ? tid : 0));
+#pragma unroll 1
+    for (int t = tid; t < B1; t += NT) {
+        const int j = jof(t);
+        cpair v[R1], m[NLO + 1];
+        czero(m[NLO]);
+#pragma unroll
+        for (int r = 0; r < R1; ++r) czero(v[r]);
+#pragma unroll
+        for (int r = 0; r < NLO; ++r) {
+            const int k = j + r * B1;
+            czero(m[r]);
+            if ((r + 1) * B1 <= H || k < H) {
+                const row2 x = ld_row2(row + (size_t)k * widx_kx_stride);
+                if (r == 0 && k == 0) {
+                    v[r] = {make_float2(x.a.x, x.b.x), make_float2(x.a.z, x.b.z)};
+                } else {
+                    v[r] = {make_float2(x.a.x - x.a.w, x.b.x - x.b.w), make_float2(x.a.y + x.a.z, x.b.y + x.b.z)};
+                }
+                m[r] = {make_float2(x.a.x + x.a.w, x.b.x + x.b.w), make_float2(x.a.z - x.a.y, x.b.z - x.b.y)};
+            }
+        }
+#pragma unroll
+        for (int r = R1 - NLO; r < R1; ++r) {
+            cpair h = shfl_xor16(m[R1 - 1 - r]);
+            if (j == 0) h = m[R1 - r];
+            else if (j == B1 / 2) h = m[R1 - 1 - r];
+            v[r] = h;
+        }
+        DFT<R1, true>::run(v);
+        ip_twiddle<R1, true>(v, w1);
+        if (t + NT < B1) ip_tw_load<Cat, R1, B1>(w1, p.tw, jof(t + NT));
+        ip_store<R1, B1>(s4, v, j ^ ((j / R3) & 7));
+    }
+    static_assert(32 % R3 == 0, "a thread's index within a block's R3 is the same in every round");
+    ip_tw_load<Cat, R2, R3>(w2, p.tw, lane % R3);
+    __syncthreads();
+#pragma unroll 1
+    for (int t = lane; t < BPW * R3; t += 32) {
+        const int i3 = t % R3, i1 = warp * BPW + t / R3;
+        const int b = i1 * B1 + (i3 ^ (i1 & 7));
+        cpair v[R2];
+        ip_load<R2, R3>(v, s4, b);
+        DFT<R2, true>::run(v);
+        ip_twiddle<R2, true>(v, w2);
+        ip_store<R2, R3>(s4, v, b);
+    }
+    __syncwarp();
+    // last inverse stage -> products (u + iw)^2 -> first forward stage, in registers
+#pragma unroll 1
+    for (int t = lane; t < BPW * R2; t += 32) {
+        const int i2 = t % R2, i1 = warp * BPW + t / R2;
+        const int b = i1 * B1 + i2 * R3 + ((i1 ^ i2) & 7);
+        cpair v[R3];
+        ip_load_run<R3>(v, s4, b);
+        DFT<R3, true>::run(v);
+#pragma unroll
+        for (int q = 0; q < R3; ++q) {
+            const float2 u = v[q].re, w = v[q].im;
+            v[q].re = __ffma2_rn(u, u, __fmul2_rn(cscale(w, -1.f), w));
+            v[q].im = __fmul2_rn(__fadd2_rn(u, u), w);
+        }
+        DFT<R3, false>::run(v);
+        ip_store_run<R3>(s4, v, b);
+    }
+    __syncwarp();
+#pragma unroll 1
+    for (int t = lane; t < BPW * R3; t += 32) {
+        const int i3 = t % R3, i1 = warp * BPW + t / R3;
+        const int b = i1 * B1 + (i3 ^ (i1 & 7));
+        cpair v[R2];
+        ip_load<R2, R3>(v, s4, b);
+        ip_twiddle<R2, false>(v, w2);
+        DFT<R2, false>::run(v);
+        ip_store<R2, R3>(s4, v, b);
+    }
+    ip_tw_load<Cat, R1, B1>(w1, p.tw, jof(tid < B1 ? tid : 0));
+    __syncthreads();
+#pragma unroll 1
+    for (int t = tid; t < B1; t += NT) {
+        const int j = jof(t);
+        cpair v[R1];
+        ip_load<R1, B1>(v, s4, j ^ ((j / R3) & 7));
+        ip_twiddle<R1, false>(v, w1);
+        if (t + NT < B1) ip_tw_load<Cat, R1, B1>(w1, p.tw, jof(t + NT));
+        DFT<R1, false>::run(v);
+        // mode k = j + r B1 < H and its mirror L - k: slot R1 - 1 - r of butterfly B1 - j
+#pragma unroll
+        for (int r = 0; r < NLO; ++r) {
+            const int k = j + r * B1;
+            cpair m = shfl_xor16(v[R1 - 1 - r]);
+            if (j == 0) m = v[r == 0 ? 0 : R1 - r];
+            else if (j == B1 / 2) m = v[R1 - 1 - r];
+            if ((r + 1) * B1 <= H || k < H) {
+                row2 o;
+                o.a = make_float4(0.5f * (v[r].re.x + m.re.x), 0.5f * (v[r].im.x - m.im.x),
+                                  0.25f * (v[r].im.x + m.im.x), -0.25f * (v[r].re.x - m.re.x));
+                o.b = make_float4(0.5f * (v[r].re.y + m.re.y), 0.5f * (v[r].im.y - m.im.y),
+                                  0.25f * (v[r].im.y + m.im.y), -0.25f * (v[r].re.y - m.re.y));
+                st_row2(row + (size_t)k * widx_kx_stride, o);
+            }
+        }
+    }
+}
+
+// ------------------------------------------------------------------------------------------
+// Column pass: column kx: D, E -> z-forward -> FN, Crank-Nicolson / AB2, FNM1 <- FN, velocity
+// recovery -> z-inverse -> U, W.  The column arrives by cp.async in natural order; a thread waits
+// only for its own copies (it copies what its first butterflies read).  In the R3 stage the threads
+// run along kz, so om2 and fnm1 are read and written coalesced; the 3/2 band's slots are zeros known
+// at compile time where they lie wholly in it.
+// ------------------------------------------------------------------------------------------
+template <int N>
+__global__ void __launch_bounds__(CfgI<N>::NTC, CfgI<N>::MBC) k_cols_ip(Pointers p0, int first, int hist_slot)
+{
+    const Pointers p = p0.member(blockIdx.y);
+    using C = CfgI<N>;
+    using P = typename C::ColPlan;
+    using Cat = TwCat<N>;
+    constexpr int L = C::L, H = C::H, NT = C::NTC, R1 = P::R1, R2 = P::R2, R3 = P::R3, B1 = P::B1;
+    constexpr int S3 = R1 * R2, NLO = (H + S3 - 1) / S3, HI0 = (L - H) / S3;
+    static_assert(HI0 + NLO == R3 && NLO <= HI0, "retained slots");
+    static_assert(B1 % 32 == 0, "whole warps in the first and last stage");
+    extern __shared__ __align__(16) float4 s4[];
+    __shared__ double2 red[NT / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int kx = blockIdx.x;
+    float2 *om2c = p.om2 + (size_t)kx * N;
+    float2 *fnc = p.fnm1 + (size_t)kx * N;
+    static_assert(B1 % widx_rows == 0, "stride");
+    constexpr size_t ZS = (size_t)(B1 / widx_rows) * H * widx_kx_stride;  // float2 between z and z + B1
+    constexpr int ND1 = (B1 + NT - 1) / NT;
+#pragma unroll
+    for (int i = 0; i < ND1; ++i) {
+        const int j = tid + i * NT;
+        if (B1 % NT == 0 || j < B1) {
+            const float2 *ptr = p.work + widx<L, H>(0, j, kx);
+#pragma unroll
+            for (int r = 0; r < R1; ++r) cp_async16(s4 + j + r * B1, ptr + r * ZS);
+        }
+        cp_async_commit();
+    }
+    for (int o = tid * 16; o < N; o += NT * 16) {
+        prefetch_l2(om2c + o);
+        prefetch_l2(fnc + o);
+    }
+    float2 w1[R1], w2[R2];
+    ip_tw_load<Cat, R1, B1>(w1, p.tw, tid < B1 ? tid : 0);
+#pragma unroll 1
+    for (int i = 0; i < ND1; ++i) {
+        const int j = tid + i * NT;
+        if (B1 % NT != 0 && j >= B1) break;
+        cpair v[R1];
+        cp_async_wait_first<ND1>(i);
+#pragma unroll
+        for (int r = 0; r < R1; ++r) {
+            const float4 x = s4[j + r * B1];
+            v[r] = {make_float2(x.x, x.z), make_float2(x.y, x.w)};
+        }
+        DFT<R1, false>::run(v);
+        ip_twiddle<R1, false>(v, w1);
+        if (j + NT < B1) ip_tw_load<Cat, R1, B1>(w1, p.tw, j + NT);
+        __syncwarp();  // the swizzled positions are other lanes' inputs
+        ip_store<R1, B1>(s4, v, j ^ ((j / R3) & 7));
+    }
+    static_assert(32 % R3 == 0, "a thread's index within a block's R3 is the same in every round");
+    ip_tw_load<Cat, R2, R3>(w2, p.tw, lane % R3);
+    __syncthreads();
+#pragma unroll 1
+    for (int t = tid; t < R1 * R3; t += NT) {
+        const int i3 = t % R3, i1 = t / R3;
+        const int b = i1 * B1 + (i3 ^ (i1 & 7));
+        cpair v[R2];
+        ip_load<R2, R3>(v, s4, b);
+        DFT<R2, false>::run(v);
+        ip_twiddle<R2, false>(v, w2);
+        ip_store<R2, R3>(s4, v, b);
+    }
+    const StepParams prm = *p.prm;
+    const float dt = prm.dt;
+    const float cnm1 = first ? prm.cnm1_first : prm.cn;
+    const double hvdt = 0.5 * (double)prm.visc * (double)dt;
+    const double c2n = 0.5 * (double)dt * (2.0 + (double)cnm1);
+    const double c3n = -0.5 * (double)dt * (double)cnm1;
+    const float divxz = (float)(1.0 / ((double)L * (double)L));
+    double2 ez = make_double2(0.0, 0.0);
+    const double wgt = (kx == 0) ? 0.5 : 1.0;
+    __syncthreads();
+#pragma unroll 1
+    for (int j = tid; j < S3; j += NT) {
+        const int i1 = j % R1, i2 = j / R1;
+        const int b = i1 * B1 + i2 * R3 + ((i1 ^ i2) & 7);
+        float2 om[2 * NLO], fo[2 * NLO];
+#pragma unroll
+        for (int q = 0; q < 2 * NLO; ++q) {
+            const int kzi = j + S3 * (q < NLO ? q : HI0 - NLO + q);
+            const int iz = q < NLO ? kzi : kzi - (L - N);
+            om[q] = fo[q] = make_float2(0.f, 0.f);
+            if (q < NLO ? kzi < H : kzi >= L - H) {
+                om[q] = om2c[iz];
+                fo[q] = fnc[iz];
+            }
+        }
+        cpair v[R3];
+        ip_load_run<R3>(v, s4, b);
+        DFT<R3, false>::run(v);
+#pragma unroll
+        for (int q = NLO; q < HI0; ++q) czero(v[q]);
+#pragma unroll
+        for (int q = 0; q < 2 * NLO; ++q) {
+            const int slot = q < NLO ? q : HI0 - NLO + q;
+            const int kzi = j + S3 * slot;
+            const int kz = q < NLO ? kzi : kzi - L, iz = q < NLO ? kzi : kzi - (L - N);
+            cpair uw;
+            czero(uw);
+            if (q < NLO ? kzi < H : kzi >= L - H) {
+                const float2 d = make_float2(v[slot].re.x, v[slot].im.x), e = make_float2(v[slot].re.y, v[slot].im.y);
+                float2 fn = make_float2(0.f, 0.f);
+                if (kz != -H) {
+                    const float ga = (float)kz * (float)kx;
+                    const float g2a2 = (float)kz * (float)kz - (float)kx * (float)kx;
+                    fn.x = (ga * d.x + g2a2 * e.x) * divxz;
+                    fn.y = (ga * d.y + g2a2 * e.y) * divxz;
+                    if (p.force) fn = add_forcing(fn, p, kx, iz, N);
+                }
+                const double K2 = (double)kx * kx + (double)kz * kz;
+                const float2 on = cn_update(om[q], fn, fo[q], K2, hvdt, c2n, c3n);
+                om2c[iz] = on;
+                fnc[iz] = fn;
+                double invK2;
+                float2 u, w;
+                recover_velocity(kx, kz, on, u, w, invK2);
+                uw = {make_float2(u.x, w.x), make_float2(u.y, w.y)};
+                const double pw = (double)on.x * on.x + (double)on.y * on.y;
+                ez.x += wgt * pw * invK2;
+                ez.y += wgt * pw;
+            }
+            v[slot] = uw;
+        }
+        DFT<R3, true>::run(v);
+        ip_store_run<R3>(s4, v, b);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        ez.x += __shfl_xor_sync(0xffffffffu, ez.x, o);
+        ez.y += __shfl_xor_sync(0xffffffffu, ez.y, o);
+    }
+    if (lane == 0) red[warp] = ez;
+    ip_tw_load<Cat, R2, R3>(w2, p.tw, lane % R3);
+    __syncthreads();
+    // energy / enstrophy: per-column partials, the last column's first warp sums them (deterministic)
+    if (warp == 0) {
+        ez = lane < NT / 32 ? red[lane] : make_double2(0.0, 0.0);
+        for (int o = 16; o > 0; o >>= 1) {
+            ez.x += __shfl_xor_sync(0xffffffffu, ez.x, o);
+            ez.y += __shfl_xor_sync(0xffffffffu, ez.y, o);
+        }
+        unsigned int n = 0;
+        if (lane == 0) {
+            p.part[kx] = ez;
+            __threadfence();
+            n = atomicAdd(p.counter, 1u);
+        }
+        n = __shfl_sync(0xffffffffu, n, 0);
+        if (n == gridDim.x - 1) {
+            __threadfence();
+            double2 acc = make_double2(0.0, 0.0);
+            for (int i = lane; i < H; i += 32) {
+                const double2 q = __ldcg(&p.part[i]);
+                acc.x += q.x;
+                acc.y += q.y;
+            }
+            for (int o = 16; o > 0; o >>= 1) {
+                acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o);
+                acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
+            }
+            if (lane == 0) {
+                p.hist[hist_slot] = acc;
+                *p.counter = 0u;
+            }
+        }
+    }
+#pragma unroll 1
+    for (int t = tid; t < R1 * R3; t += NT) {
+        const int i3 = t % R3, i1 = t / R3;
+        const int b = i1 * B1 + (i3 ^ (i1 & 7));
+        cpair v[R2];
+        ip_load<R2, R3>(v, s4, b);
+        ip_twiddle<R2, true>(v, w2);
+        DFT<R2, true>::run(v);
+        ip_store<R2, R3>(s4, v, b);
+    }
+    ip_tw_load<Cat, R1, B1>(w1, p.tw, tid < B1 ? tid : 0);
+    __syncthreads();
+#pragma unroll 1
+    for (int j = tid; j < B1; j += NT) {
+        cpair v[R1];
+        ip_load<R1, B1>(v, s4, j ^ ((j / R3) & 7));
+        ip_twiddle<R1, true>(v, w1);
+        if (j + NT < B1) ip_tw_load<Cat, R1, B1>(w1, p.tw, j + NT);
+        DFT<R1, true>::run(v);
+        float4 *ptr = reinterpret_cast<float4 *>(p.work + widx<L, H>(0, j, kx));
+#pragma unroll
+        for (int r = 0; r < R1; ++r) ptr[r * (ZS / 2)] = make_float4(v[r].re.x, v[r].im.x, v[r].re.y, v[r].im.y);
+    }
+}
+
+}  // namespace dns2d

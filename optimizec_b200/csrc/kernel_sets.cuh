@@ -5,6 +5,7 @@
 #pragma once
 #include "dns2d_kernels.cuh"
 #include "cluster.cuh"
+#include "inplace.cuh"
 
 namespace dns2d {
 
@@ -41,6 +42,7 @@ struct Launch {
 
     static constexpr bool V2 = Cfg2<N>::enabled;
     static constexpr size_t sm2 = V2 ? (size_t)Cfg2<N>::LP * sizeof(float2) : 0;
+    static constexpr size_t smI = (size_t)C::L * 2 * sizeof(float2);  // two interleaved arrays, no padding
     using P0 = typename C::Plan;
     using P1 = typename AltPlans<N>::P1;
     using P2 = typename AltPlans<N>::P2;
@@ -74,9 +76,8 @@ struct Launch {
         const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
         cudaError_t e;
         if constexpr (V2) {
-            if ((e = cudaFuncSetAttribute(k_rows_step2<N>, a, (int)sm2)) != cudaSuccess) return e;
-            if ((e = cudaFuncSetAttribute(k_cols_step2<N>, a, (int)(2 * sm2))) != cudaSuccess) return e;
-            if ((e = cudaFuncSetAttribute(k_cols_step4<N>, a, (int)cols4_smem_bytes<N>())) != cudaSuccess) return e;
+            if ((e = cudaFuncSetAttribute(k_rows_ip<N>, a, (int)smI)) != cudaSuccess) return e;
+            if ((e = cudaFuncSetAttribute(k_cols_ip<N>, a, (int)smI)) != cudaSuccess) return e;
             if ((e = cudaFuncSetAttribute(k_rows_velocity2<N>, a, (int)sm2)) != cudaSuccess) return e;
             if ((e = cudaFuncSetAttribute(k_cols_scalar2<N>, a, (int)sm2)) != cudaSuccess) return e;
             if ((e = cudaFuncSetAttribute(k_rows_pair2<N>, a, (int)sm2)) != cudaSuccess) return e;
@@ -86,7 +87,6 @@ struct Launch {
             if ((e = setup_plan<P1>()) != cudaSuccess) return e;
             if ((e = setup_plan<P2>()) != cudaSuccess) return e;
         }
-        if ((e = cudaFuncSetAttribute(k_cols_step<N>, a, (int)smA)) != cudaSuccess) return e;
         if ((e = cudaFuncSetAttribute(k_cols_init<N>, a, (int)smA)) != cudaSuccess) return e;
         if ((e = cudaFuncSetAttribute(k_rows_velocity<N>, a, (int)smB)) != cudaSuccess) return e;
         if ((e = cudaFuncSetAttribute(k_rows_from_phys<N>, a, (int)smB)) != cudaSuccess) return e;
@@ -101,7 +101,7 @@ struct Launch {
     static void rows_step(const Pointers &p, cudaStream_t s, int ny)
     {
         if constexpr (V2) {
-            k_rows_step2<N><<<dim3(C::L, ny), Cfg2<N>::NT, sm2, s>>>(p);
+            k_rows_ip<N><<<dim3(C::L / 2, ny), CfgI<N>::NTR, smI, s>>>(p);
         } else {
             if (p.plan_rows == 1) rows_plan<P1>(p, s, ny);
             else if (p.plan_rows == 2) rows_plan<P2>(p, s, ny);
@@ -110,13 +110,7 @@ struct Launch {
     }
     static void cols_step(const Pointers &p, int first, int slot, cudaStream_t s, int ny)
     {
-        // one or two thread groups per column CTA (autotuned; the default, two, was the faster on
-        // B200 at N = 1024, 2048 and 4096); both give the same arithmetic
-        if constexpr (V2) {
-            const int g = p.cols_groups ? p.cols_groups : 2;
-            if (g == 2) k_cols_step4<N><<<dim3(C::H, ny), 2 * Cfg2<N>::NT, cols4_smem_bytes<N>(), s>>>(p, first, slot);
-            else k_cols_step2<N><<<dim3(C::H, ny), Cfg2<N>::NT, 2 * sm2, s>>>(p, first, slot);
-        }
+        if constexpr (V2) k_cols_ip<N><<<dim3(C::H, ny), CfgI<N>::NTC, smI, s>>>(p, first, slot);
         else if (p.plan_cols == 1) k_cols_step<N, P1><<<dim3(C::H, ny), C::NTA, smA, s>>>(p, first, slot);
         else if (p.plan_cols == 2) k_cols_step<N, P2><<<dim3(C::H, ny), C::NTA, smA, s>>>(p, first, slot);
         else k_cols_step<N, P0><<<dim3(C::H, ny), C::NTA, smA, s>>>(p, first, slot);
