@@ -69,6 +69,10 @@ constexpr TwCatalog make_catalog_c()
     c.add(typename CfgC<N>::Plan{});
     const int cross[] = {CfgC<N>::M, 4};  // adds the stage (4, Ns = M): W_L^{r m}, r = 1..3
     c.add_plan(cross, 2);
+    if constexpr (CfgI<N>::enabled) {
+        c.add(typename CfgI<N>::RowPlan::Tw{});
+        c.add(typename CfgI<N>::ColPlan::Tw{});
+    }
     return c;
 }
 

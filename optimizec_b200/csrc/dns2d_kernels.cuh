@@ -496,11 +496,15 @@ struct CfgI {
 // thread counts divide a stage's L / R butterflies into whole rounds where they can.  Other
 // choices measured on B200 (rows, columns in us): 4096 rows 256 threads 201, columns 128 threads 217,
 // 256 threads 217, plan (24, 32, 8) 226; 2048 rows 64 threads 55.5, columns (16, 12, 16) 55, rows
-// (16, 24, 8) 54.5; 1024 (few CTAs per SM: more threads each) 64 threads 21.6 / 25.8.
+// (16, 24, 8) 54.5; 1024 (few CTAs per SM: more threads each) 64 threads 21.6 / 25.8.  8192 and 9216
+// fit one CTA per SM: 8192 rows (32, 24, 16) 944, 512 threads 1076, columns (32, 24, 16) 883, (16, 24, 32)
+// 1160; 9216 rows (24, 36, 16) 1418, (18, 24, 32) 1457, columns (16, 27, 32) 1304, (36, 24, 16) 1416.
 //          N     rows: NT MB  plan        columns: NT MB  plan
 DNS2D_CFGI(1024,      128, 4, 16, 12, 8,           128, 4, 16, 12, 8)
 DNS2D_CFGI(2048,      128, 4, 16, 12, 16,          128, 4, 16, 24, 8)
 DNS2D_CFGI(4096,      128, 2, 16, 24, 16,          192, 2, 16, 24, 16)
+DNS2D_CFGI(8192,      256, 1, 16, 24, 32,          384, 1, 24, 32, 16)
+DNS2D_CFGI(9216,      256, 1, 16, 27, 32,          384, 1, 24, 36, 16)
 #undef DNS2D_CFGI
 
 // twiddle catalog of size N: the stages of every plan compiled for it

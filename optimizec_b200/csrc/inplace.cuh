@@ -26,15 +26,22 @@
 // by the latency of its phases at two CTAs per SM (HBM 35 %, issue 32 %).  Measured (rows / columns,
 // one launch): N = 4096 0.254 / 0.293 -> 0.186 / 0.211 ms, N = 2048 67.6 / 71.7 -> 50.8 / 51.0 us,
 // N = 1024 27.0 / 28.2 -> 20.1 / 23.6 us against the auto-sort kernels that these replace (one row,
-// or one array and thread group, per 384 threads).
+// or one array and thread group, per 384 threads).  N = 8192 2.08 / 1.52 -> 0.88 / 0.86 ms and N = 9216
+// 2.99 / 2.11 -> 1.25 / 1.26 ms against the 4-CTA cluster kernels: two rows or one kx fill an SM's
+// shared memory (192 / 216 KB), and no sequence crosses CTAs.
 // Tried and slower, or no faster: each sequence on its own lane with scalar butterflies (rows 0.185,
 // columns 0.223 ms at N = 4096), fetching the next round's twiddles, state or rows into registers
 // (columns 0.220-0.239 ms), prefetching a later CTA's input to L2 (columns +4 us), twice the threads at
 // half the registers (rows 0.200 ms), 2-row tiles of the work buffer (columns 0.259 ms).
 #pragma once
-#include "dns2d_kernels.cuh"
+#include "cluster.cuh"
 
 namespace dns2d {
+
+// twiddle catalog of a size with in-place passes
+template <int N>
+using IpCat = std::conditional_t<CfgC<N>::enabled, TwCatC<N>, TwCat<N>>;
+
 
 // shared-memory element <-> the two complex values of a butterfly input
 __device__ __forceinline__ cpair ip_get(const float4 *s, int i)
@@ -133,7 +140,7 @@ __global__ void __launch_bounds__(CfgI<N>::NTR, CfgI<N>::MBR) k_rows_ip(Pointers
     const Pointers p = p0.member(blockIdx.y);
     using C = CfgI<N>;
     using P = typename C::RowPlan;
-    using Cat = TwCat<N>;
+    using Cat = IpCat<N>;
     constexpr int L = C::L, H = C::H, NT = C::NTR, R1 = P::R1, R2 = P::R2, R3 = P::R3, B1 = P::B1;
     constexpr int NW = NT / 32, BPW = R1 / NW;  // blocks of B1 elements per warp
     static_assert(R1 % NW == 0 && B1 % 32 == 0, "whole blocks per warp");
@@ -141,6 +148,12 @@ __global__ void __launch_bounds__(CfgI<N>::NTR, CfgI<N>::MBR) k_rows_ip(Pointers
     extern __shared__ __align__(16) float4 s4[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     float2 *__restrict__ row = p.work + widx<L, H>(0, 2 * blockIdx.x, 0);
+    // one CTA per SM: nothing else runs while its rows arrive, so the rows of a later CTA are brought to
+    // L2 (N = 8192 / 9216: rows 0.898 / 1.309 -> 0.881 / 1.251 ms; the column pass gained nothing)
+    if (C::MBR == 1 && (int)blockIdx.x + 74 < L / 2) {
+        const float2 *nx = p.work + widx<L, H>(0, 2 * ((int)blockIdx.x + 74), 0);
+        for (int k = tid; k < H; k += NT) prefetch_l2(nx + (size_t)k * widx_kx_stride);
+    }
     auto jof = [](int t) {  // butterfly of index t
         const int l = t & 31, q = (t >> 5) * 16 + (l & 15);
         return (l < 16) ? q : (q == 0 ? B1 / 2 : B1 - q);
@@ -264,7 +277,7 @@ __global__ void __launch_bounds__(CfgI<N>::NTC, CfgI<N>::MBC) k_cols_ip(Pointers
     const Pointers p = p0.member(blockIdx.y);
     using C = CfgI<N>;
     using P = typename C::ColPlan;
-    using Cat = TwCat<N>;
+    using Cat = IpCat<N>;
     constexpr int L = C::L, H = C::H, NT = C::NTC, R1 = P::R1, R2 = P::R2, R3 = P::R3, B1 = P::B1;
     constexpr int S3 = R1 * R2, NLO = (H + S3 - 1) / S3, HI0 = (L - H) / S3;
     static_assert(HI0 + NLO == R3 && NLO <= HI0, "retained slots");

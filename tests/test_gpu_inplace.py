@@ -6,7 +6,7 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-SIZES = [1024, 2048, 4096]
+SIZES = [1024, 2048, 4096, 8192, 9216]
 
 
 def P():
