@@ -1,4 +1,6 @@
-// cnn_gemm.cuh — the closure network's training convolutions on the 5th-gen tensor cores.
+// cnn_gemm.cuh — the closure network's training convolutions on the 5th-gen tensor cores, for image
+// widths that are no multiple of 16 and for the closure's own evaluation of a network in training mode
+// (the other widths: cnn_train.cuh).
 //
 // Every 3x3 periodic convolution of training is one skinny GEMM with N = 32 (padded) on tcgen05,
 // BF16 operands and FP32 accumulators in tensor memory, fed by an explicit im2col expansion:

@@ -178,20 +178,27 @@ __device__ __forceinline__ void mma_commit(uint64_t *mbar)
                  : "memory");
 }
 
-// wait (at most kWaitNs) for the phase of the given parity to complete; false when it ran out
+__device__ __forceinline__ bool mbar_try(uint64_t *mbar, uint32_t parity)
+{
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(done)
+        : "r"(saddr(mbar)), "r"(parity)
+        : "memory");
+    return done != 0;
+}
+
+// wait (at most kWaitNs) for the phase of the given parity to complete; false when it ran out.  The
+// timer is read only once a first try (which itself waits a while) has failed.
 __device__ __forceinline__ bool mbar_wait(uint64_t *mbar, uint32_t parity)
 {
-    uint32_t done = 0;
+    if (mbar_try(mbar, parity)) return true;
     const unsigned long long t0 = global_ns();
-    for (;;) {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
-            : "=r"(done)
-            : "r"(saddr(mbar)), "r"(parity)
-            : "memory");
-        if (done || global_ns() - t0 > kWaitNs) break;
-    }
-    return done != 0;
+    do {
+        if (mbar_try(mbar, parity)) return true;
+    } while (global_ns() - t0 <= kWaitNs);
+    return false;
 }
 
 __device__ __forceinline__ void mbar_init(uint64_t *m, uint32_t count)

@@ -18,6 +18,7 @@
 #include "ensemble.cuh"
 #include "cnn.cuh"
 #include "cnn_gemm.cuh"
+#include "cnn_train.cuh"
 #include "cnn_net.cuh"
 #include "cnn_tc.cuh"
 #include "../../include/dns2d.h"
@@ -2627,6 +2628,8 @@ struct dns2d_cnn {
     int trace_on = 0, trace_tiles = 0;
     // training convolutions as tcgen05 GEMMs (cnn_gemm.cuh) when train_tc is set
     dns2d::cnngemm::Work gw;
+    // the same on chunk planes, without im2col expansions (cnn_train.cuh), where the width allows it
+    dns2d::cnntrain::Planes planes;
     int train_tc = 0;
     long long gen = 0, tc_gen = -1;
     std::string err;
@@ -2691,10 +2694,41 @@ void conv(dns2d_cnn *n, const float *x, const float *w, const float *b, float *y
     k_conv3x3<<<grid, dim3(TILE, TILE), sm, st>>>(x, w, b, y, B, Ci, Co, H, W);
 }
 
+// training on chunk planes: tensor-core training on, and a width whose rows are whole K steps of the
+// weight gradient (other widths take the im2col GEMMs of cnn_gemm.cuh)
+bool train_planes(const dns2d_cnn *n, int H, int W)
+{
+    return n->train_tc && dns2d::cnntrain::supported(n->channels, H, W);
+}
+
+dns2d::cnntrain::Net train_net(dns2d_cnn *n, int B, int H, int W)
+{
+    dns2d::cnntrain::Net t;
+    t.L = n->layers;
+    t.B = B;
+    t.H = H;
+    t.W = W;
+    t.ci = n->ci.data();
+    t.co = n->co.data();
+    t.woff = n->woff.data();
+    t.params = n->params;
+    t.grad = n->grad;
+    t.x = n->xin;
+    t.z = n->z.data();
+    t.dout = n->gout;
+    return t;
+}
+
 // forward of B images in n->xin; output (layer L-1 pre-activation) in n->z[L-1]
 int cnn_forward_dev(dns2d_cnn *n, int B, int H, int W, cudaStream_t st = nullptr)
 {
-    if (!st) st = n->stream;
+    if (!st) {
+        st = n->stream;
+        if (train_planes(n, H, W)) {
+            CNN_CUDA(dns2d::cnntrain::forward(train_net(n, B, H, W), n->planes, st), "tensor-core forward");
+            return DNS2D_OK;
+        }
+    }
     const float *in = n->xin;
     if (n->train_tc) {  // every layer as a tcgen05 GEMM (bf16 operands, FP32 accumulation)
         for (int l = 0; l < n->layers; ++l) {
@@ -2757,8 +2791,6 @@ int cnn_tc_reserve(dns2d_cnn *n, int B, int H, int W)
     if (words > n->net_sync_cap) {
         CNN_CUDA(cudaStreamSynchronize(n->stream), "sync");
         cudaFree(n->net_sync);
-    cudaFree(n->trace);
-    dns2d::cnngemm::work_free(n->gw);
         n->net_sync = nullptr;
         CNN_CUDA(cudaMalloc((void **)&n->net_sync, words * 4), "network counters alloc");
         CNN_CUDA(cudaMemset(n->net_sync, 0, words * 4), "network counters clear");
@@ -2844,6 +2876,10 @@ int cnn_forward_tc_dev(dns2d_cnn *n, int B, int H, int W, const dns2d::cnntc::Fi
 // backward from the loss gradient in n->gout (shape of the output); fills n->grad
 int cnn_backward_dev(dns2d_cnn *n, int B, int H, int W)
 {
+    if (train_planes(n, H, W)) {
+        CNN_CUDA(dns2d::cnntrain::backward(train_net(n, B, H, W), n->planes, n->stream), "tensor-core backward");
+        return DNS2D_OK;
+    }
     float *dz = n->gout, *other = n->gtmp;
     if (n->train_tc && ((size_t)B * H * W) % dns2d::cnngemm::BK == 0) {
         // weight and data gradients as tcgen05 GEMMs; GELU' is applied in the data-gradient epilogue
@@ -2923,6 +2959,8 @@ extern "C" void dns2d_cnn_destroy(dns2d_cnn *n)
     cudaFree(n->tc_err);
     cudaFree(n->net_sync);
     cudaFree(n->trace);
+    dns2d::cnngemm::work_free(n->gw);
+    dns2d::cnntrain::release(n->planes);
     if (n->stream) cudaStreamDestroy(n->stream);
     delete n;
 }
@@ -3054,11 +3092,12 @@ extern "C" int dns2d_cnn_set_train_tc(dns2d_cnn *n, int on)
 // the tensor-core training GEMMs' wait flag (0 when no GEMM ran); the stream is synchronised
 static int train_tc_status(dns2d_cnn *n)
 {
-    if (!n->gw.err) return DNS2D_OK;
-    int flag = 0;
-    CNN_CUDA(cudaMemcpyAsync(&flag, n->gw.err, 4, cudaMemcpyDeviceToHost, n->stream), "flag copy");
+    int flag[2] = {0, 0};
+    if (n->gw.err) CNN_CUDA(cudaMemcpyAsync(flag, n->gw.err, 4, cudaMemcpyDeviceToHost, n->stream), "flag copy");
+    if (n->planes.err)
+        CNN_CUDA(cudaMemcpyAsync(flag + 1, n->planes.err, 4, cudaMemcpyDeviceToHost, n->stream), "flag copy");
     CNN_CUDA(cudaStreamSynchronize(n->stream), "flag sync");
-    if (flag) return nfail(n, DNS2D_ERR_TIMEOUT, "tensor-core training GEMM wait timed out");
+    if (flag[0] || flag[1]) return nfail(n, DNS2D_ERR_TIMEOUT, "tensor-core training GEMM wait timed out");
     return DNS2D_OK;
 }
 
@@ -3145,12 +3184,14 @@ extern "C" int dns2d_cnn_train(dns2d_cnn *n, int iters, int batch, float lr, uin
             const int j = i + (int)(sm64(st) % (uint64_t)(n->data_n - i));
             std::swap(idx[(size_t)i], idx[(size_t)j]);
         }
-        for (int i = 0; i < batch; ++i) {
-            const int k = idx[(size_t)(i % n->data_n)];
-            CNN_CUDA(cudaMemcpyAsync(n->xin + i * xs, n->data_x + k * xs, xs * 4, cudaMemcpyDeviceToDevice, n->stream),
-                     "batch gather");
-            CNN_CUDA(cudaMemcpyAsync(n->tgt + i * ts, n->data_t + k * ts, ts * 4, cudaMemcpyDeviceToDevice, n->stream),
-                     "batch gather");
+        // the minibatch, kGather samples of it per launch
+        for (int i0 = 0; i0 < batch; i0 += dns2d::cnn::kGather) {
+            dns2d::cnn::GatherIdx g;
+            g.n = std::min(dns2d::cnn::kGather, batch - i0);
+            for (int i = 0; i < g.n; ++i) g.src[i] = idx[(size_t)((i0 + i) % n->data_n)];
+            dns2d::cnn::k_gather<<<dim3((unsigned)std::min<size_t>(256, (xs + ts + 1023) / 1024), g.n), 256, 0, n->stream>>>(
+                n->data_x, n->data_t, g, n->xin + i0 * xs, n->tgt + i0 * ts, xs, ts);
+            CNN_CUDA(cudaGetLastError(), "batch gather");
         }
         double loss = 0.0;
         if ((rc = cnn_forward_dev(n, batch, H, W)) || (rc = cnn_loss(n, batch, H, W, losses ? &loss : nullptr)) ||
