@@ -1,4 +1,5 @@
 // cnn_train.cu — training convolutions on chunk planes (cnn_train.cuh).
+#include "cnn_math.cuh"
 #include "cnn_train.cuh"
 #include "cnn_tc.cuh"
 
@@ -21,12 +22,8 @@ using cnntc::saddr;
 using cnntc::smem_desc;
 using cnntc::tmem_ld32;
 
-// the same GELU and derivative as the FP32 path (erf form)
-__device__ __forceinline__ float gelu(float z) { return 0.5f * z * (1.0f + erff(z * 0.70710678118654752f)); }
-__device__ __forceinline__ float gelu_grad(float z)
-{
-    return 0.5f * (1.0f + erff(z * 0.70710678118654752f)) + z * 0.39894228040143268f * expf(-0.5f * z * z);
-}
+using cnn::gelu;
+using cnn::gelu_grad;
 
 __device__ __forceinline__ uint4 pack8(const float *v)
 {
@@ -470,14 +467,13 @@ __global__ void __launch_bounds__(kWgradThreads, 1) k_wgrad_planes(const __grid_
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(128));
 }
 
-// dw[co][ci][tap] and db[co] from the G partials: one CTA per row of an accumulator, 8 warps over g
-// (lane = column; output channel co in column c0 + co), FP64 in fixed order.  Row m: of the planes of one
+// dw[co][ci][tap] and db[co] from the G partials: one CTA per row of an accumulator (output channel
+// co in column c0 + co).  Row m: of the planes of one
 // kernel row after another, or (rows 1) the products k = tap Ci + ci of a point tensor; row 8 x planes: db.
 __global__ void __launch_bounds__(256) k_reduce_planes(const float *__restrict__ part, int G, int rows, int nchi, int c0,
                                                        int Ci, int Co, float *__restrict__ dw, float *__restrict__ db)
 {
-    __shared__ double red[8][32];
-    const int m = blockIdx.x, dx = blockIdx.y, lane = threadIdx.x & 31, w = threadIdx.x >> 5, co = lane - c0;
+    const int m = blockIdx.x, dx = blockIdx.y, co = (threadIdx.x & 31) - c0;
     const bool ones = m == 8 * rows * nchi;
     int tap, ci;
     if (rows == 3) {
@@ -489,14 +485,8 @@ __global__ void __launch_bounds__(256) k_reduce_planes(const float *__restrict__
         ci = m - tap * Ci;
     }
     if (ones ? dx != 0 : (ci >= Ci || tap >= 9)) return;
-    double s = 0.0;
-#pragma unroll 4
-    for (int g = w; g < G; g += 8) s += (double)__ldg(part + (((size_t)g * rows + dx) * 128 + m) * 32 + lane);
-    red[w][lane] = s;
-    __syncthreads();
-    if (w != 0 || co < 0 || co >= Co) return;
-#pragma unroll
-    for (int i = 1; i < 8; ++i) s += red[i][lane];
+    const double s = cnn::sum_partials(part + ((size_t)dx * 128 + m) * 32, G, (size_t)rows * 128 * 32);
+    if (threadIdx.x >= 32 || co < 0 || co >= Co) return;
     if (ones) db[co] = (float)s;
     else dw[((size_t)co * Ci + ci) * 9 + tap] = (float)s;
 }

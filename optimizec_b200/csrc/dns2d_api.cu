@@ -2602,9 +2602,12 @@ struct dns2d_cnn {
     std::vector<int> ci, co;       // per layer
     std::vector<size_t> woff;      // weight offset per layer (bias follows the weights)
     cudaStream_t stream = nullptr;
-    float *params = nullptr, *grad = nullptr, *adam_m = nullptr, *adam_v = nullptr, *wflip = nullptr, *zero = nullptr;
+    float *params = nullptr, *grad = nullptr, *adam_m = nullptr, *adam_v = nullptr;
     std::vector<float *> z, a;     // pre-activations / activations per layer (capacity cap_elems each)
     float *xin = nullptr, *tgt = nullptr, *gout = nullptr, *gtmp = nullptr;
+    float *wg_part = nullptr;      // partial sums of the FP32 weight gradient
+    float *wpack = nullptr;        // packed weights of the FP32 convolutions, per layer forward and data gradient
+    std::vector<size_t> pk_fwd, pk_bwd;
     size_t cap_elems = 0;          // per activation tensor: B * max(C, 3) * H * W
     int capB = 0, capH = 0, capW = 0;
     double *part = nullptr;
@@ -2685,13 +2688,41 @@ int cnn_reserve(dns2d_cnn *n, int B, int H, int W)
     return DNS2D_OK;
 }
 
-void conv(dns2d_cnn *n, const float *x, const float *w, const float *b, float *y, int B, int Ci, int Co, int H, int W,
-          cudaStream_t st)
+// one FP32 convolution (cnn.cuh) with packed weights; few output channels take the tile of 8
+void conv(const float *x, const float *w, const float *bias, const float *zprev, float *y, float *a, int B, int Ci, int Co,
+          int H, int W, cudaStream_t st)
 {
     using namespace dns2d::cnn;
-    dim3 grid((W + TILE - 1) / TILE, (H + TILE - 1) / TILE, B * ((Co + COT - 1) / COT));
-    const size_t sm = ((size_t)Ci * (TILE + 2) * (TILE + 2) + (size_t)COT * Ci * 9) * 4;
-    k_conv3x3<<<grid, dim3(TILE, TILE), sm, st>>>(x, w, b, y, B, Ci, Co, H, W);
+    const int tx = (W + kConvCols - 1) / kConvCols, NP = packed_channels(Co);
+    if (Co <= 8)
+        k_conv3x3<1><<<dim3(tx * ((H + kConvRows<1> - 1) / kConvRows<1>), 1, B), kConvThreads, conv_smem<1>(), st>>>(
+            x, w, bias, zprev, y, a, Ci, Co, H, W, NP);
+    else
+        k_conv3x3<4><<<dim3(tx * ((H + kConvRows<4> - 1) / kConvRows<4>), NP / 32, B), kConvThreads, conv_smem<4>(), st>>>(
+            x, w, bias, zprev, y, a, Ci, Co, H, W, NP);
+}
+
+// packed FP32 weights of every layer into n->wpack
+void pack_fp32(dns2d_cnn *n, cudaStream_t st)
+{
+    for (int l0 = 0; l0 < n->layers; l0 += dns2d::cnn::kPackLayers) {
+        dns2d::cnn::PackFp32 a;
+        const int L = std::min(dns2d::cnn::kPackLayers, n->layers - l0);
+        for (int i = 0; i < L; ++i) {
+            a.ci[i] = n->ci[l0 + i];
+            a.co[i] = n->co[l0 + i];
+            a.woff[i] = (unsigned)n->woff[l0 + i];
+            a.fwd[i] = (unsigned)n->pk_fwd[l0 + i];
+            a.bwd[i] = (unsigned)n->pk_bwd[l0 + i];
+        }
+        dns2d::cnn::k_pack_fp32<<<dim3(8, 2 * L), 256, 0, st>>>(n->params, a, n->wpack);
+    }
+}
+
+// CTAs of the FP32 weight gradient per channel tile: two per SM in all
+int wgrad_ctas(int tiles, long long units)
+{
+    return (int)std::max<long long>(1, std::min<long long>(units, 148 * dns2d::cnn::kWgCtas / tiles));
 }
 
 // training on chunk planes: tensor-core training on, and a width whose rows are whole K steps of the
@@ -2740,14 +2771,15 @@ int cnn_forward_dev(dns2d_cnn *n, int B, int H, int W, cudaStream_t st = nullptr
         }
         return DNS2D_OK;
     }
+    pack_fp32(n, st);
     for (int l = 0; l < n->layers; ++l) {
-        conv(n, in, n->params + n->woff[l], n->params + n->woff[l] + (size_t)n->co[l] * n->ci[l] * 9, n->z[l], B,
-             n->ci[l], n->co[l], H, W, st);
-        if (l + 1 < n->layers) {
-            const size_t cnt = (size_t)B * n->co[l] * H * W;
-            dns2d::cnn::k_gelu<<<1024, 256, 0, st>>>(n->z[l], n->a[l], cnt);
-            in = n->a[l];
-        }
+        const float *bias = n->params + n->woff[l] + (size_t)n->co[l] * n->ci[l] * 9;
+        if (l + 1 == n->layers)  // one output channel
+            dns2d::cnn::k_conv3x3_one<<<dim3((W * H + 127) / 128, B), 128, (size_t)n->ci[l] * 9 * sizeof(float), st>>>(
+                in, n->params + n->woff[l], bias, n->z[l], n->ci[l], H, W);
+        else
+            conv(in, n->wpack + n->pk_fwd[l], bias, nullptr, n->z[l], n->a[l], B, n->ci[l], n->co[l], H, W, st);
+        in = n->a[l];
     }
     CNN_CUDA(cudaGetLastError(), "cnn forward");
     return DNS2D_OK;
@@ -2898,17 +2930,18 @@ int cnn_backward_dev(dns2d_cnn *n, int B, int H, int W)
         }
         return DNS2D_OK;
     }
+    pack_fp32(n, n->stream);  // a forward in tensor-core mode leaves them unpacked
     for (int l = n->layers - 1; l >= 0; --l) {
         const float *xin = (l == 0) ? n->xin : n->a[l - 1];
         float *dw = n->grad + n->woff[l];
         float *db = dw + (size_t)n->co[l] * n->ci[l] * 9;
-        dns2d::cnn::k_conv3x3_wgrad<<<dim3(n->ci[l], n->co[l]), 256, 0, n->stream>>>(xin, dz, dw, db, B, n->ci[l],
-                                                                                   n->co[l], H, W);
+        const int tiles = ((n->ci[l] + 31) / 32) * ((n->co[l] + 31) / 32);
+        const int G = wgrad_ctas(tiles, (long long)B * H * ((W + dns2d::cnn::kWgCols - 1) / dns2d::cnn::kWgCols));
+        dns2d::cnn::k_conv3x3_wgrad<<<dim3(G, tiles), dns2d::cnn::kWgThreads, dns2d::cnn::wgrad_smem(), n->stream>>>(
+            xin, dz, n->wg_part, B, n->ci[l], n->co[l], H, W);
+        dns2d::cnn::k_wgrad_reduce<<<dim3(9 * 32 + 1, tiles), 256, 0, n->stream>>>(n->wg_part, G, dw, db, n->ci[l], n->co[l]);
         if (l > 0) {
-            dns2d::cnn::k_flip_weights<<<64, 256, 0, n->stream>>>(n->params + n->woff[l], n->wflip, n->ci[l], n->co[l]);
-            conv(n, dz, n->wflip, n->zero, other, B, n->co[l], n->ci[l], H, W, n->stream);
-            const size_t cnt = (size_t)B * n->ci[l] * H * W;
-            dns2d::cnn::k_gelu_back<<<1024, 256, 0, n->stream>>>(n->z[l - 1], other, cnt);
+            conv(dz, n->wpack + n->pk_bwd[l], nullptr, n->z[l - 1], other, nullptr, B, n->co[l], n->ci[l], H, W, n->stream);
             std::swap(dz, other);
         }
     }
@@ -2944,8 +2977,8 @@ extern "C" void dns2d_cnn_destroy(dns2d_cnn *n)
     cudaFree(n->grad);
     cudaFree(n->adam_m);
     cudaFree(n->adam_v);
-    cudaFree(n->wflip);
-    cudaFree(n->zero);
+    cudaFree(n->wg_part);
+    cudaFree(n->wpack);
     cudaFree(n->xin);
     cudaFree(n->tgt);
     cudaFree(n->gout);
@@ -3001,20 +3034,27 @@ extern "C" int dns2d_cnn_create(dns2d_cnn **out, int layers, int channels, uint6
             p[n->woff[l] + i] = (float)(sd * std::sqrt(-2.0 * std::log(u1)) * std::cos(2.0 * M_PI * u2));
         }
     }
-    size_t maxw = 0;
-    for (int l = 0; l < layers; ++l) maxw = std::max(maxw, (size_t)n->co[l] * n->ci[l] * 9);
+    size_t pk = 0;
+    for (int l = 0; l < layers; ++l) {
+        n->pk_fwd.push_back(pk);
+        pk += (size_t)n->ci[l] * 9 * dns2d::cnn::packed_channels(n->co[l]);
+        n->pk_bwd.push_back(pk);
+        pk += (size_t)n->co[l] * 9 * dns2d::cnn::packed_channels(n->ci[l]);
+    }
+    const int ct = (channels + 31) / 32, tiles = ct * ct;
+    const size_t wg = (size_t)tiles * wgrad_ctas(tiles, 1ll << 30) * dns2d::cnn::kWgPart;
     if (cudaMalloc((void **)&n->params, off * 4) != cudaSuccess || cudaMalloc((void **)&n->grad, off * 4) != cudaSuccess ||
         cudaMalloc((void **)&n->adam_m, off * 4) != cudaSuccess || cudaMalloc((void **)&n->adam_v, off * 4) != cudaSuccess ||
-        cudaMalloc((void **)&n->wflip, maxw * 4) != cudaSuccess || cudaMalloc((void **)&n->zero, 256 * 4) != cudaSuccess ||
-        cudaMalloc((void **)&n->part, 256 * 8) != cudaSuccess)
+        cudaMalloc((void **)&n->wg_part, std::max(wg, (size_t)148 * dns2d::cnn::kWgCtas * dns2d::cnn::kWgPart) * 4) != cudaSuccess ||
+        cudaMalloc((void **)&n->wpack, pk * 4) != cudaSuccess || cudaMalloc((void **)&n->part, 256 * 8) != cudaSuccess)
         return bail(DNS2D_ERR_NOMEM);
     if (cudaMemcpy(n->params, p.data(), off * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemset(n->adam_m, 0, off * 4) != cudaSuccess || cudaMemset(n->adam_v, 0, off * 4) != cudaSuccess ||
-        cudaMemset(n->zero, 0, 256 * 4) != cudaSuccess)
+        cudaMemset(n->adam_m, 0, off * 4) != cudaSuccess || cudaMemset(n->adam_v, 0, off * 4) != cudaSuccess)
         return bail(DNS2D_ERR_CUDA);
-    const int smax = (int)(((size_t)channels * (dns2d::cnn::TILE + 2) * (dns2d::cnn::TILE + 2) +
-                            (size_t)dns2d::cnn::COT * channels * 9) * 4);
-    if (cudaFuncSetAttribute(dns2d::cnn::k_conv3x3, cudaFuncAttributeMaxDynamicSharedMemorySize, smax) != cudaSuccess)
+    const cudaFuncAttribute sm = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    if (cudaFuncSetAttribute(dns2d::cnn::k_conv3x3<1>, sm, (int)dns2d::cnn::conv_smem<1>()) != cudaSuccess ||
+        cudaFuncSetAttribute(dns2d::cnn::k_conv3x3<4>, sm, (int)dns2d::cnn::conv_smem<4>()) != cudaSuccess ||
+        cudaFuncSetAttribute(dns2d::cnn::k_conv3x3_wgrad, sm, (int)dns2d::cnn::wgrad_smem()) != cudaSuccess)
         return bail(DNS2D_ERR_CUDA);
     *out = n;
     return DNS2D_OK;
