@@ -69,17 +69,13 @@ constexpr TwCatalog make_catalog_c()
     c.add(typename CfgC<N>::Plan{});
     const int cross[] = {CfgC<N>::M, 4};  // adds the stage (4, Ns = M): W_L^{r m}, r = 1..3
     c.add_plan(cross, 2);
-    if constexpr (CfgI<N>::enabled) {
-        c.add(typename CfgI<N>::RowPlan::Tw{});
-        c.add(typename CfgI<N>::ColPlan::Tw{});
-    }
     return c;
 }
 
 template <int N>
 struct TwCatC {
     static constexpr TwCatalog cat = make_catalog_c<N>();
-    static constexpr int off(int R, int NS) { return cat.find(R, NS); }
+    static constexpr int off(int R, int NS, int outer = 0) { return cat.find(R, NS, outer); }
 };
 
 // W_L^{r m} (forward sign) from the cross stage table, r = 1..3

@@ -467,10 +467,11 @@ std::vector<float2> twiddles(const TwCatalog &c)
     for (int i = 0; i < c.n; ++i) {
         const int R = c.R[i], NS = c.NS[i], M = R * NS;
         for (int r = 1; r < R; ++r)
-            for (int k = 0; k < NS; ++k) {
+            for (int e = 0; e < NS; ++e) {
+                const int k = c.index(i, e);
                 const long long m = ((long long)r * k) % M;
                 const double a = 2.0 * M_PI * (double)m / (double)M;
-                t[(size_t)c.off[i] + (size_t)(r - 1) * NS + k] = make_float2((float)std::cos(a), (float)-std::sin(a));
+                t[(size_t)c.off[i] + (size_t)(r - 1) * NS + e] = make_float2((float)std::cos(a), (float)-std::sin(a));
             }
     }
     return t;
@@ -3608,7 +3609,7 @@ __global__ void k_noalloc_twiddles(float2 *tw, TwCatalog c)
         while (i + 1 < c.n && c.off[i + 1] <= e) ++i;
         const int R = c.R[i], NS = c.NS[i], M = R * NS;
         const int loc = e - c.off[i];
-        const int r = loc / NS + 1, k = loc % NS;
+        const int r = loc / NS + 1, k = c.index(i, loc);
         const long long m = ((long long)r * k) % M;
         double sn, cs;
         sincospi(2.0 * (double)m / (double)M, &sn, &cs);

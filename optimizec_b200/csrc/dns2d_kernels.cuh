@@ -145,9 +145,9 @@ struct Pointers {
     size_t s_state, s_work;
     int s_part, s_hist;
     // kernel configuration (the autotuner's choice; every choice gives the same arithmetic):
-    // rows per CTA of the small-grid row pass (0: the size's default)
+    // rows per CTA of k_rows_step (0: the size's default; the in-place pass takes two)
     int rows_tile = 0;
-    // radix plan of the small-grid row / column pass (0: Cfg<N>::Plan, 1, 2: AltPlans<N>); unlike
+    // radix plan of the small-grid row / column pass (0: the default, 1, 2: AltPlans<N>); unlike
     // the knobs above a plan changes the FP32 rounding
     int plan_rows = 0, plan_cols = 0;
     // closure forcing limiter: |forcing| <= force_clamp |FN| per mode (0: off)
@@ -467,14 +467,20 @@ DNS2D_CFG2(2048, 256, 16, 12, 16, 4)
 DNS2D_CFG2(4096, 384, 16, 24, 16, 4)
 #undef DNS2D_CFG2
 
-// Radix plan of an in-place transform (inplace.cuh); its forward half has the twiddle stages of the
-// auto-sort plan (R3, R2, R1).
+// Radix plan of an in-place transform (inplace.cuh): the first transform of a pass computes what the
+// auto-sort plan (R1, R2, R3) does, the second what (R3, R2, R1) does.
 template <int L_, int R1_, int R2_, int R3_>
 struct InPlan {
     static constexpr int L = L_, R1 = R1_, R2 = R2_, R3 = R3_, B1 = R2_ * R3_;
     static_assert(R1_ * R2_ * R3_ == L_, "plan");
     static_assert(R3_ % 8 == 0 && B1 % 32 == 0, "swizzle groups of 8, whole warps in the R1 stage");
-    using Tw = Radices<R3_, R2_, R1_>;
+    // transposed: the last stage's twiddles in the order of a thread's digits i1 (R2) + i2 (row pass)
+    static constexpr void add_twiddles(TwCatalog &c, bool transposed)
+    {
+        c.add_stage(R2, R1);
+        c.add_stage(R3, R1 * R2, transposed ? R1 : 0);
+        c.add(Radices<R3, R2, R1>{});
+    }
 };
 
 template <int N_>
@@ -493,18 +499,14 @@ struct CfgI {
     };
 // Threads per CTA, CTAs per SM asked of the register allocator and plan (R1, R2, R3), rows then
 // columns.  Shared memory (16 L bytes) allows 2 / 4 / 8 CTAs per SM at N = 4096 / 2048 / 1024; the
-// thread counts divide a stage's L / R butterflies into whole rounds where they can.  Other
-// choices measured on B200 (rows, columns in us): 4096 rows 256 threads 201, columns 128 threads 217,
-// 256 threads 217, plan (24, 32, 8) 226; 2048 rows 64 threads 55.5, columns (16, 12, 16) 55, rows
-// (16, 24, 8) 54.5; 1024 (few CTAs per SM: more threads each) 64 threads 21.6 / 25.8.  8192 and 9216
-// fit one CTA per SM: 8192 rows (32, 24, 16) 944, 512 threads 1076, columns (32, 24, 16) 883, (16, 24, 32)
-// 1160; 9216 rows (24, 36, 16) 1418, (18, 24, 32) 1457, columns (16, 27, 32) 1304, (36, 24, 16) 1416.
+// thread counts divide a stage's L / R butterflies into whole rounds where they can.  2048 and 4096 keep
+// the radices of the large-grid plans (Cfg2) and so their rounding.  Other choices measured on B200 (us):
+// 4096 columns 128 threads 218, one CTA of 384 threads 234; 2048 columns 192 threads 59.5 (58.6), 96 threads
+// 60.0; 1024 columns (8, 12, 16) with 96 threads 25.1 (23.2).
 //          N     rows: NT MB  plan        columns: NT MB  plan
-DNS2D_CFGI(1024,      128, 4, 16, 12, 8,           128, 4, 16, 12, 8)
-DNS2D_CFGI(2048,      128, 4, 16, 12, 16,          128, 4, 16, 24, 8)
+DNS2D_CFGI(1024,      128, 4, 16, 12, 8,            128, 4, 16, 12, 8)
+DNS2D_CFGI(2048,      128, 4, 16, 12, 16,          128, 4, 16, 12, 16)
 DNS2D_CFGI(4096,      128, 2, 16, 24, 16,          192, 2, 16, 24, 16)
-DNS2D_CFGI(8192,      256, 1, 16, 24, 32,          384, 1, 24, 32, 16)
-DNS2D_CFGI(9216,      256, 1, 16, 27, 32,          384, 1, 24, 36, 16)
 #undef DNS2D_CFGI
 
 // twiddle catalog of size N: the stages of every plan compiled for it
@@ -522,8 +524,8 @@ constexpr TwCatalog make_catalog()
         c.add(Radices<Cfg2<N>::R3, Cfg2<N>::R2, Cfg2<N>::R1>{});
     }
     if constexpr (CfgI<N>::enabled) {
-        c.add(typename CfgI<N>::RowPlan::Tw{});
-        c.add(typename CfgI<N>::ColPlan::Tw{});
+        CfgI<N>::RowPlan::add_twiddles(c, true);
+        CfgI<N>::ColPlan::add_twiddles(c, false);
     }
     return c;
 }
@@ -531,7 +533,7 @@ constexpr TwCatalog make_catalog()
 template <int N>
 struct TwCat {
     static constexpr TwCatalog cat = make_catalog<N>();
-    static constexpr int off(int R, int NS) { return cat.find(R, NS); }
+    static constexpr int off(int R, int NS, int outer = 0) { return cat.find(R, NS, outer); }
 };
 
 // Inverse x transform of a row pair on the large-grid plan: the half spectra A = U[k], B = W[k]
@@ -601,7 +603,7 @@ __device__ __forceinline__ void rows_inverse2(const float2 *__restrict__ U, cons
                 }
             }
         }
-        DFT<R1, true>::run(v);
+        dft_scalar<R1, true>(v);
         sm_store<L, R1, 1, PS>(s, v, jb);
     }
     stage1<TwCat<N>, L, R2, R1, true, PS>(s, tw);
@@ -644,7 +646,7 @@ __device__ __forceinline__ void stage1g_first_band(float2 *s, const float2 *tw, 
 #pragma unroll
         for (int r = 0; r < R; ++r)
             v[r] = slot_in_band<L, R, B0, B1>(r) ? make_float2(0.f, 0.f) : s[sidx<PS>(j + r * LR)];
-        DFT<R, INV>::run(v);
+        dft_scalar<R, INV>(v);
     }
     group_sync<NTH>(bar);
     if (j < LR) sm_store<L, R, 1, PS>(s, v, j);
@@ -794,7 +796,9 @@ __global__ void __launch_bounds__(Cfg<N>::NTA) k_cols_init(Pointers p0, const fl
         sW[sidx<PS>(z)] = make_float2(0.f, 0.f);
     }
     __syncthreads();
-    fft_run<TwCat<N>, L, LP, true, 2, NT, PS>(smem, p.tw, typename C::Plan{});
+    // the large-grid sizes keep the rounding of their set-up and diagnostics (see cscalar)
+    using V = std::conditional_t<Cfg2<N>::enabled, cscalar, float2>;
+    fft_run<TwCat<N>, L, LP, true, 2, NT, PS, false, V>(smem, p.tw, typename C::Plan{});
     for (int z = threadIdx.x; z < L; z += NT) {
         p.work[widx<L, H>(0, z, kx)] = sU[sidx<PS>(z)];
         p.work[widx<L, H>(1, z, kx)] = sW[sidx<PS>(z)];

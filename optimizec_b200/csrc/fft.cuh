@@ -75,16 +75,12 @@ __device__ __forceinline__ void static_for(F &&f)
 // ------------------------------------------------------------------------------------------
 // complex helpers
 // ------------------------------------------------------------------------------------------
-// Additions and scalings of both parts are one packed FP32 instruction (two results for one issue
-// slot; the butterflies are mostly additions): N = 256 / 512 step 12.5 / 22.3 -> 11.6 / 20.4 us, the
-// 64-member ensemble 130 -> 120 us per step on B200.
+// Additions, scalings and rotations of both parts are packed FP32 instructions (two results for one issue
+// slot; the butterflies are mostly additions): N = 256 / 512 step 12.5 / 22.3 -> 12.0 / 20.6 us, the
+// 64-member ensemble 130 -> 125 us per step on B200, with the rounding of the scalar expressions (see crot).
 __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 csub(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
-__device__ __forceinline__ float2 cmul(float2 a, float2 b)
-{
-    const float2 t = __fmul2_rn(a, make_float2(b.x, b.x));
-    return make_float2(fmaf(-a.y, b.y, t.x), fmaf(a.x, b.y, t.y));
-}
+__device__ __forceinline__ float2 cmul(float2 a, float2 b) { return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); }
 __device__ __forceinline__ float2 cconj(float2 a) { return make_float2(a.x, -a.y); }
 __device__ __forceinline__ float2 cscale(float2 a, float s) { return __fmul2_rn(a, make_float2(s, s)); }
 // multiply by -i (forward) or +i (inverse)
@@ -108,11 +104,21 @@ __device__ __forceinline__ float2 cfma_mi(float2 t, float f, float2 m)
     return INV ? make_float2(fmaf(-t.y, f, m.x), fmaf(t.x, f, m.y)) : make_float2(fmaf(t.y, f, m.x), fmaf(-t.x, f, m.y));
 }
 // a (c + i s)
-__device__ __forceinline__ float2 crot(float2 a, float c, float s) { return cmul(a, make_float2(c, s)); }
+//
+// Which of its two products an FMA rounds is fixed here so that the results equal, bit for bit, those of
+// the scalar expression (a.x c - a.y s, a.x s + a.y c) as the compiler contracts it: the real part keeps
+// a.x c exact, the imaginary part a.x s, or (ALT) a.y c where the sum is written as a difference.
+template <bool ALT = false>
+__device__ __forceinline__ float2 crot(float2 a, float c, float s)
+{
+    if (ALT) return __ffma2_rn(a, make_float2(c, c), __fmul2_rn(make_float2(a.y, a.x), make_float2(-s, s)));
+    return __ffma2_rn(make_float2(a.x, a.x), make_float2(c, s), __fmul2_rn(make_float2(a.y, a.y), make_float2(-s, c)));
+}
 __device__ __forceinline__ void czero(float2 &a) { a = make_float2(0.f, 0.f); }
 
-// A complex value whose operations are written one part at a time, for the compiler to contract as it
-// likes: the 4-CTA cluster kernels keep the rounding of their results this way.
+// A complex value whose operations are written one part at a time, for the compiler to contract: the
+// 4-CTA cluster kernels (radices that the packed forms below were not compared for) and the large-grid
+// diagnostics.
 struct cscalar {
     float x, y;
 };
@@ -136,6 +142,7 @@ __device__ __forceinline__ cscalar cfma_mi(cscalar t, float f, cscalar m)
 {
     return cadd(m, cmul_mi<INV>(cscale(t, f)));
 }
+template <bool ALT = false>
 __device__ __forceinline__ cscalar crot(cscalar a, float c, float s)
 {
     return {a.x * c - a.y * s, a.x * s + a.y * c};
@@ -157,11 +164,11 @@ __device__ __forceinline__ cpair cfma_mi(cpair t, float f, cpair m)
 {
     return INV ? cpair{cfma(t.im, -f, m.re), cfma(t.re, f, m.im)} : cpair{cfma(t.im, f, m.re), cfma(t.re, -f, m.im)};
 }
+template <bool ALT = false>
 __device__ __forceinline__ cpair crot(cpair a, float c, float s)
 {
-    return {cfma(a.im, -s, cscale(a.re, c)), cfma(a.re, s, cscale(a.im, c))};
+    return {cfma(a.re, c, cscale(a.im, -s)), ALT ? cfma(a.im, c, cscale(a.re, s)) : cfma(a.re, s, cscale(a.im, c))};
 }
-__device__ __forceinline__ cpair cmul(cpair a, float2 w) { return crot(a, w.x, w.y); }
 template <bool INV>
 __device__ __forceinline__ cpair cmul_mi(cpair a)
 {
@@ -174,10 +181,37 @@ __device__ __forceinline__ cpair cadd_mi(cpair a, cpair b)
     if constexpr (INV) return {csub(a.re, b.im), cadd(a.im, b.re)};
     else return {cadd(a.re, b.im), csub(a.im, b.re)};
 }
+// the squares (u + i w)^2 = u^2 - w^2 + 2 i u w of a pair, the imaginary part as its two factors: the sum or
+// difference of two is one rounding fewer, a FMA on one product (again as the compiler contracts the
+// scalar expressions)
+struct csquare {
+    float2 re, u2, w;
+};
+__device__ __forceinline__ csquare square(cpair a)
+{
+    return {__ffma2_rn(a.re, a.re, __fmul2_rn(cscale(a.im, -1.f), a.im)), cadd(a.re, a.re), a.im};
+}
+__device__ __forceinline__ cpair cadd(csquare a, csquare b)
+{
+    return {cadd(a.re, b.re), __ffma2_rn(a.u2, a.w, __fmul2_rn(b.u2, b.w))};
+}
+__device__ __forceinline__ cpair csub(csquare a, csquare b)
+{
+    return {csub(a.re, b.re), __ffma2_rn(a.u2, a.w, __fmul2_rn(cscale(b.u2, -1.f), b.w))};
+}
 __device__ __forceinline__ void czero(cpair &a) { a = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)}; }
 
-// a * W_R^K with W_R = exp(-+ 2 pi i / R); trivial angles become sign swaps
-template <int R, int K, bool INV, class V>
+// a w (forward) or a conj(w) (inverse): the twiddles before a butterfly
+template <bool INV, class V>
+__device__ __forceinline__ V ctwiddle(V a, float2 w)
+{
+    if constexpr (std::is_same_v<V, cscalar>) return cmul(a, INV ? cconj(w) : w);
+    else return INV ? crot<true>(a, w.x, -w.y) : crot(a, w.x, w.y);
+}
+
+// a * W_R^K with W_R = exp(-+ 2 pi i / R); trivial angles become sign swaps.  SWAP: the other order of the
+// imaginary part's sum (see crot; where |c| = |s| the compiler shares the products and has one order).
+template <int R, int K, bool INV, bool SWAP = false, class V>
 __device__ __forceinline__ V twid(V a)
 {
     constexpr int k = ((K % R) + R) % R;
@@ -192,7 +226,7 @@ __device__ __forceinline__ V twid(V a)
     } else {
         constexpr float c = (float)ct_cos(k, R);
         constexpr float s = INV ? (float)ct_sin(k, R) : -(float)ct_sin(k, R);
-        return crot(a, c, s);
+        return crot<c != s && c != -s && (c > 0.f && s < 0.f) != SWAP>(a, c, s);
     }
 }
 
@@ -240,8 +274,13 @@ struct DFT<4, INV> {
     template <class V>
     static __device__ __forceinline__ void run(V (&v)[4])
     {
-        const V t0 = cadd(v[0], v[2]), t1 = csub(v[0], v[2]);
-        const V t2 = cadd(v[1], v[3]), t3 = csub(v[1], v[3]);
+        run(v, v);
+    }
+    template <class In, class V>
+    static __device__ __forceinline__ void run(const In (&x)[4], V (&v)[4])
+    {
+        const V t0 = cadd(x[0], x[2]), t1 = csub(x[0], x[2]);
+        const V t2 = cadd(x[1], x[3]), t3 = csub(x[1], x[3]);
         v[0] = cadd(t0, t2);
         v[2] = csub(t0, t2);
         v[1] = cadd_mi<INV>(t1, t3);
@@ -286,27 +325,48 @@ struct DFTGeneric<R, INV, true> {
     }
 };
 
+template <int SWAP_N2, int R, bool INV, class V>
+__device__ __forceinline__ void dft_swapped(V (&v)[R])
+{
+    if constexpr (SWAP_N2 > 0) DFTGeneric<R, INV>::template run<SWAP_N2>(v);
+    else DFT<R, INV>::run(v);
+}
+
 // composite R = P * Q, decimation in time:
 // X[k1 + P k2] = sum_{n2} W_R^{n2 k1} W_Q^{n2 k2} sum_{n1} x[Q n1 + n2] W_P^{n1 k1}
 template <int R, bool INV>
 struct DFTGeneric<R, INV, false> {
-    template <class V>
+    // SWAP_N2: a pair whose rotations take the other order of crot in the place that this transform has in a
+    // larger one; the rotations of i t differences (INV, P = 4, odd k1) always do
+    template <int SWAP_N2 = 0, class V>
     static __device__ __forceinline__ void run(V (&v)[R])
+    {
+        run<SWAP_N2>(v, v);
+    }
+    template <int SWAP_N2 = 0, class In, class V>
+    static __device__ __forceinline__ void run(const In (&x)[R], V (&v)[R])
     {
         constexpr int P = ct_first_factor(R);
         constexpr int Q = R / P;
         V t[R];
         static_for<0, Q>([&](auto n2c) {
             constexpr int n2 = decltype(n2c)::value;
+            In b[P];
             V a[P];
             static_for<0, P>([&](auto n1c) {
                 constexpr int n1 = decltype(n1c)::value;
-                a[n1] = v[Q * n1 + n2];
+                b[n1] = x[Q * n1 + n2];
             });
-            DFT<P, INV>::run(a);
+            if constexpr (std::is_same_v<In, V>) {
+                static_for<0, P>([&](auto n1c) { a[decltype(n1c)::value] = b[decltype(n1c)::value]; });
+                DFT<P, INV>::run(a);
+            } else {
+                DFT<P, INV>::run(b, a);
+            }
             static_for<0, P>([&](auto k1c) {
                 constexpr int k1 = decltype(k1c)::value;
-                t[k1 * Q + n2] = twid<R, n2 * k1, INV>(a[k1]);
+                constexpr bool SWAP = (INV && P == 4 && k1 % 2 == 1) != (SWAP_N2 > 0 && n2 == SWAP_N2);
+                t[k1 * Q + n2] = twid<R, n2 * k1, INV, SWAP>(a[k1]);
             });
         });
         static_for<0, P>([&](auto k1c) {
@@ -316,7 +376,7 @@ struct DFTGeneric<R, INV, false> {
                 constexpr int n2 = decltype(n2c)::value;
                 b[n2] = t[k1 * Q + n2];
             });
-            DFT<Q, INV>::run(b);
+            dft_swapped<R == 24 && INV && k1 == 3 ? 1 : 0, Q, INV>(b);
             static_for<0, Q>([&](auto k2c) {
                 constexpr int k2 = decltype(k2c)::value;
                 v[k1 + P * k2] = b[k2];
@@ -331,6 +391,11 @@ struct DFT {
     static __device__ __forceinline__ void run(V (&v)[R])
     {
         DFTGeneric<R, INV>::run(v);
+    }
+    template <class In, class V>
+    static __device__ __forceinline__ void run(const In (&x)[R], V (&v)[R])
+    {
+        DFTGeneric<R, INV>::run(x, v);
     }
 };
 
@@ -375,23 +440,34 @@ struct TwCatalog {
     int R[64] = {};
     int NS[64] = {};
     int off[64] = {};
-    constexpr int find(int r, int ns) const
+    int outer[64] = {};  // P > 0: index k = i1 + P i2 is stored at i1 (NS / P) + i2
+    constexpr int find(int r, int ns, int p = 0) const
     {
         for (int i = 0; i < n; ++i)
-            if (R[i] == r && NS[i] == ns) return off[i];
+            if (R[i] == r && NS[i] == ns && outer[i] == p) return off[i];
         return -1;
+    }
+    constexpr void add_stage(int r, int ns, int p = 0)
+    {
+        if (find(r, ns, p) >= 0) return;
+        R[n] = r;
+        NS[n] = ns;
+        outer[n] = p;
+        off[n] = total;
+        total += (r - 1) * ns;
+        ++n;
+    }
+    // power k of entry `loc` of stage i (its r is loc / NS + 1)
+    __host__ __device__ constexpr int index(int i, int loc) const
+    {
+        const int e = loc % NS[i], p = outer[i], w = p ? NS[i] / p : 1;
+        return p ? e / w + p * (e % w) : e;
     }
     constexpr void add_plan(const int *rs, int nr)
     {
         int ns = 1;
         for (int i = 0; i < nr; ++i) {
-            if (ns > 1 && find(rs[i], ns) < 0) {
-                R[n] = rs[i];
-                NS[n] = ns;
-                off[n] = total;
-                total += (rs[i] - 1) * ns;
-                ++n;
-            }
+            if (ns > 1) add_stage(rs[i], ns);
             ns *= rs[i];
         }
     }
@@ -441,9 +517,7 @@ __device__ __forceinline__ void fft_stage(float2 *__restrict__ s, const float2 *
                 const float2 *t = tw + OFF + j % NS;
 #pragma unroll
                 for (int r = 1; r < R; ++r) {
-                    float2 w = __ldg(t + (r - 1) * NS);
-                    if constexpr (INV) w.y = -w.y;
-                    v[i][r] = cmul(v[i][r], w);
+                    v[i][r] = ctwiddle<INV>(v[i][r], __ldg(t + (r - 1) * NS));
                 }
             }
             DFT<R, INV>::run(v[i]);
@@ -472,6 +546,17 @@ __device__ __forceinline__ void fft_stage(float2 *__restrict__ s, const float2 *
 // reads of the first stage can come straight from global memory, and the last stage's outputs
 // (Ns = L/R: positions j + q L/R) can go straight back, skipping two shared-memory passes.
 // ------------------------------------------------------------------------------------------
+template <int R, bool INV>
+__device__ __forceinline__ void dft_scalar(float2 (&v)[R])
+{
+    cscalar c[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) c[r] = {v[r].x, v[r].y};
+    DFT<R, INV>::run(c);
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = make_float2(c[r].x, c[r].y);
+}
+
 template <class Cat, int L, int R, int NS, bool INV>
 __device__ __forceinline__ void bfly(float2 (&v)[R], int j, const float2 *__restrict__ tw)
 {
@@ -483,10 +568,11 @@ __device__ __forceinline__ void bfly(float2 (&v)[R], int j, const float2 *__rest
         for (int r = 1; r < R; ++r) {
             float2 w = __ldg(t + (r - 1) * NS);
             if constexpr (INV) w.y = -w.y;
-            v[r] = cmul(v[r], w);
+            const cscalar c = cmul(cscalar{v[r].x, v[r].y}, w);
+            v[r] = make_float2(c.x, c.y);
         }
     }
-    DFT<R, INV>::run(v);
+    dft_scalar<R, INV>(v);
 }
 
 // 1: shared-memory addresses of a butterfly as one base plus compile-time offsets where the
@@ -598,8 +684,7 @@ __device__ __forceinline__ void fft_stages(float2 *s, const float2 *tw)
     if constexpr (sizeof...(Rs) > 0) fft_stages<V, Cat, L, LP, INV, B, NT, PS, OPQ, NS * R0, Rs...>(s, tw);
 }
 
-// PS: the padding of sidx<PS>; OPQ: read the thread index with opaque_tid(); V: the type a complex
-// value is computed in
+// PS: the padding of sidx<PS>; OPQ: read the thread index with opaque_tid(); V: the type a complex value is computed in
 template <class Cat, int L, int LP, bool INV, int B, int NT, int PS = 5, bool OPQ = false, class V = float2, int... Rs>
 __device__ __forceinline__ void fft_run(float2 *s, const float2 *tw, Radices<Rs...>)
 {

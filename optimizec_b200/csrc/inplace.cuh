@@ -8,9 +8,8 @@
 // Every stage is in place: a butterfly writes its outputs to the positions its inputs came from,
 // so nothing is held in registers across a barrier and one barrier separates two stages (the
 // auto-sort stages of fft.cuh need two, and the registers of all threads in between).  The first
-// transform of a pass runs natural -> digit-reversed order (decimation in frequency: radix R1 over
-// the L/R1-strided digit, then R2, then R3 over R3 contiguous elements), the second one
-// digit-reversed -> natural (decimation in time, R3, R2, R1), and what lies between the two (the
+// transform of a pass runs natural -> digit-reversed order (radix R1 over the L/R1-strided digit, then
+// R2, then R3 over R3 contiguous elements), the second one digit-reversed -> natural (R3, R2, R1), and what lies between the two (the
 // products of the row pass, the spectral update of the column pass) works in any order.  So no
 // reordering pass exists, and the R3 stages of both transforms with everything between them run in
 // registers: a pass touches shared memory 4 times in each direction.
@@ -21,27 +20,30 @@
 // (no CTA barrier: two per pass in all).  Bank conflicts: i3 is stored as i3 ^ ((i1 ^ i2) & 7), so
 // eight neighbouring lanes find eight different 16-byte columns in every stage, along i3, i2 or i1.
 //
+// Rounding: both transforms compute node by node what auto-sort plans do (decimation in time: twiddles
+// before a butterfly), and the packed operations round where the scalar expressions of those plans round
+// (fft.cuh), so that with the plans (16, 12, 16) and (16, 24, 16), the same in both directions, N = 2048
+// and 4096 have the auto-sort kernels' results bit for bit.  It matters: FP32 rounding of the products, times
+// k^2, is 1e-3 of the field's RMS in single modes of the corners, and a run compared with an earlier one
+// would show it.  A first transform by decimation in frequency (twiddles after a butterfly, fetched once)
+// was 1-9 % faster (N = 4096 386 us per step, 2048 89.7; here 392, 98), N = 8192 / 9216 on three-stage in-place
+// passes twice as fast as the clusters (1.75 / 2.55 ms), N = 512 and 256 15.3 and 10.6 us (20.6 and 12.1) and the
+// 64-member ensemble 77 us per step (125): all with other rounding, further from an earlier run than two runs may be.
+//
 // Bounds (N = 4096 on B200, 1965 MHz; ncu): the row pass is bound by the L1 / shared-memory data
 // pipe (67-75 % of its cycles busy; 24 % before the loads' and twiddles' share fell), the column pass
 // by the latency of its phases at two CTAs per SM (HBM 35 %, issue 32 %).  Measured (rows / columns,
-// one launch): N = 4096 0.254 / 0.293 -> 0.186 / 0.211 ms, N = 2048 67.6 / 71.7 -> 50.8 / 51.0 us,
-// N = 1024 27.0 / 28.2 -> 20.1 / 23.6 us against the auto-sort kernels that these replace (one row,
-// or one array and thread group, per 384 threads).  N = 8192 2.08 / 1.52 -> 0.88 / 0.86 ms and N = 9216
-// 2.99 / 2.11 -> 1.25 / 1.26 ms against the 4-CTA cluster kernels: two rows or one kx fill an SM's
-// shared memory (192 / 216 KB), and no sequence crosses CTAs.
+// one launch): N = 4096 0.254 / 0.293 -> 0.193 / 0.211 ms, N = 2048 67.6 / 71.7 -> 52.1 / 58.6 us,
+// N = 1024 27.0 / 28.2 -> 20.3 / 23.2 us against the auto-sort kernels that these replace (one row,
+// or one array and thread group, per 384 threads).
 // Tried and slower, or no faster: each sequence on its own lane with scalar butterflies (rows 0.185,
-// columns 0.223 ms at N = 4096), fetching the next round's twiddles, state or rows into registers
-// (columns 0.220-0.239 ms), prefetching a later CTA's input to L2 (columns +4 us), twice the threads at
+// columns 0.223 ms at N = 4096), fetching the next round's twiddles, state or rows into registers in the
+// column pass (0.220-0.239 ms), prefetching a later CTA's input to L2 (columns +4 us), twice the threads at
 // half the registers (rows 0.200 ms), 2-row tiles of the work buffer (columns 0.259 ms).
 #pragma once
-#include "cluster.cuh"
+#include "dns2d_kernels.cuh"
 
 namespace dns2d {
-
-// twiddle catalog of a size with in-place passes
-template <int N>
-using IpCat = std::conditional_t<CfgC<N>::enabled, TwCatC<N>, TwCat<N>>;
-
 
 // shared-memory element <-> the two complex values of a butterfly input
 __device__ __forceinline__ cpair ip_get(const float4 *s, int i)
@@ -80,11 +82,11 @@ __device__ __forceinline__ void ip_store_run(float4 *s, const cpair (&v)[R], int
     for (int r = 0; r < R; ++r) ip_put(s, (b ^ (r & 7)) + (r & ~7), v[r]);
 }
 
-// w[r] = W^{r k}, r >= 1: the twiddles of the stage (R, NS) at index k
-template <class Cat, int R, int NS>
+// w[r] = W^{r k}, r >= 1: the twiddles of the stage (R, NS) at index k of the table's order
+template <class Cat, int R, int NS, int OUTER = 0>
 __device__ __forceinline__ void ip_tw_load(float2 (&w)[R], const float2 *__restrict__ tw, int k)
 {
-    constexpr int OFF = Cat::off(R, NS);
+    constexpr int OFF = Cat::off(R, NS, OUTER);
     static_assert(OFF >= 0, "stage missing from the twiddle catalog");
     const float2 *t = tw + OFF + k;
 #pragma unroll
@@ -96,7 +98,7 @@ template <int R, bool INV>
 __device__ __forceinline__ void ip_twiddle(cpair (&v)[R], const float2 (&w)[R])
 {
 #pragma unroll
-    for (int r = 1; r < R; ++r) v[r] = cmul(v[r], INV ? cconj(w[r]) : w[r]);
+    for (int r = 1; r < R; ++r) v[r] = ctwiddle<INV>(v[r], w[r]);
 }
 
 // the two components of one mode on two neighbouring rows: 32 contiguous bytes of the work buffer
@@ -128,38 +130,34 @@ __device__ __forceinline__ cpair shfl_xor16(cpair m)
 }
 
 // ------------------------------------------------------------------------------------------
-// Row pass: rows 2 blockIdx.x and + 1: U, W -> C2R -> (u + iw)^2 -> R2C -> D, E.
+// Row pass by NT threads (tid < NT): rows 2 pair and + 1: U, W -> C2R -> (u + iw)^2 -> R2C -> D, E.
 // The Hermitian packing needs modes k and L - k together: k = j + r B1 is slot r of butterfly j, and
 // L - k is slot R1 - 1 - r of butterfly B1 - j, so butterflies j and B1 - j run 16 lanes apart in one
 // warp and exchange those slots by shuffle, on the way in and on the way out (butterflies 0 and
 // B1 / 2 are their own mirrors).
 // ------------------------------------------------------------------------------------------
-template <int N>
-__global__ void __launch_bounds__(CfgI<N>::NTR, CfgI<N>::MBR) k_rows_ip(Pointers p0)
+template <int N, int NT>
+__device__ __forceinline__ void rows_ip(const Pointers &p, int pair, float4 *s4, int tid)
 {
-    const Pointers p = p0.member(blockIdx.y);
     using C = CfgI<N>;
     using P = typename C::RowPlan;
-    using Cat = IpCat<N>;
-    constexpr int L = C::L, H = C::H, NT = C::NTR, R1 = P::R1, R2 = P::R2, R3 = P::R3, B1 = P::B1;
+    using Cat = TwCat<N>;
+    constexpr int L = C::L, H = C::H, R1 = P::R1, R2 = P::R2, R3 = P::R3, B1 = P::B1;
     constexpr int NW = NT / 32, BPW = R1 / NW;  // blocks of B1 elements per warp
     static_assert(R1 % NW == 0 && B1 % 32 == 0, "whole blocks per warp");
     constexpr int NLO = (H + B1 - 1) / B1;  // slots with retained modes below H
-    extern __shared__ __align__(16) float4 s4[];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    float2 *__restrict__ row = p.work + widx<L, H>(0, 2 * blockIdx.x, 0);
-    // one CTA per SM: nothing else runs while its rows arrive, so the rows of a later CTA are brought to
-    // L2 (N = 8192 / 9216: rows 0.898 / 1.309 -> 0.881 / 1.251 ms; the column pass gained nothing)
-    if (C::MBR == 1 && (int)blockIdx.x + 74 < L / 2) {
-        const float2 *nx = p.work + widx<L, H>(0, 2 * ((int)blockIdx.x + 74), 0);
-        for (int k = tid; k < H; k += NT) prefetch_l2(nx + (size_t)k * widx_kx_stride);
-    }
+    const int lane = tid & 31, warp = tid >> 5;
+    float2 *row = p.work + widx<L, H>(0, 2 * pair, 0);
     auto jof = [](int t) {  // butterfly of index t
         const int l = t & 31, q = (t >> 5) * 16 + (l & 15);
         return (l < 16) ? q : (q == 0 ? B1 / 2 : B1 - q);
     };
-    float2 w1[R1], w2[R2];
-    ip_tw_load<Cat, R1, B1>(w1, p.tw, jof(tid < B1 ? tid : 0));
+    // a round's twiddles on their way before the round, where a thread has the registers (N = 4096: rows
+    // 198 -> 193 us; 2048 and 1024, at 128 registers, 52.5 -> 53.7 and 20.6 -> 20.8)
+    constexpr bool AHEAD = 65536 / (C::MBR * C::NTR) >= 255;
+    float2 w1[R1], w2[R2], w3[R3];
+    auto first_w2 = [&] { ip_tw_load<Cat, R2, R1>(w2, p.tw, warp * BPW + (lane < BPW * R3 ? lane / R3 : 0)); };
+    auto first_w3 = [&] { ip_tw_load<Cat, R3, R1 * R2, R1>(w3, p.tw, warp * BPW * R2 + (lane < BPW * R2 ? lane : 0)); };
 #pragma unroll 1
     for (int t = tid; t < B1; t += NT) {
         const int j = jof(t);
@@ -189,23 +187,23 @@ __global__ void __launch_bounds__(CfgI<N>::NTR, CfgI<N>::MBR) k_rows_ip(Pointers
             v[r] = h;
         }
         DFT<R1, true>::run(v);
-        ip_twiddle<R1, true>(v, w1);
-        if (t + NT < B1) ip_tw_load<Cat, R1, B1>(w1, p.tw, jof(t + NT));
         ip_store<R1, B1>(s4, v, j ^ ((j / R3) & 7));
     }
-    static_assert(32 % R3 == 0, "a thread's index within a block's R3 is the same in every round");
-    ip_tw_load<Cat, R2, R3>(w2, p.tw, lane % R3);
+    if constexpr (AHEAD) first_w2();
     __syncthreads();
 #pragma unroll 1
     for (int t = lane; t < BPW * R3; t += 32) {
         const int i3 = t % R3, i1 = warp * BPW + t / R3;
         const int b = i1 * B1 + (i3 ^ (i1 & 7));
         cpair v[R2];
+        if (!AHEAD) ip_tw_load<Cat, R2, R1>(w2, p.tw, i1);
         ip_load<R2, R3>(v, s4, b);
-        DFT<R2, true>::run(v);
         ip_twiddle<R2, true>(v, w2);
+        if (AHEAD && t + 32 < BPW * R3) ip_tw_load<Cat, R2, R1>(w2, p.tw, warp * BPW + (t + 32) / R3);
+        DFT<R2, true>::run(v);
         ip_store<R2, R3>(s4, v, b);
     }
+    if constexpr (AHEAD) first_w3();
     __syncwarp();
     // last inverse stage -> products (u + iw)^2 -> first forward stage, in registers
 #pragma unroll 1
@@ -213,17 +211,19 @@ __global__ void __launch_bounds__(CfgI<N>::NTR, CfgI<N>::MBR) k_rows_ip(Pointers
         const int i2 = t % R2, i1 = warp * BPW + t / R2;
         const int b = i1 * B1 + i2 * R3 + ((i1 ^ i2) & 7);
         cpair v[R3];
+        if (!AHEAD) ip_tw_load<Cat, R3, R1 * R2, R1>(w3, p.tw, i1 * R2 + i2);
         ip_load_run<R3>(v, s4, b);
+        ip_twiddle<R3, true>(v, w3);
+        if (AHEAD && t + 32 < BPW * R2) ip_tw_load<Cat, R3, R1 * R2, R1>(w3, p.tw, warp * BPW * R2 + t + 32);
         DFT<R3, true>::run(v);
+        csquare sq[R3];
 #pragma unroll
-        for (int q = 0; q < R3; ++q) {
-            const float2 u = v[q].re, w = v[q].im;
-            v[q].re = __ffma2_rn(u, u, __fmul2_rn(cscale(w, -1.f), w));
-            v[q].im = __fmul2_rn(__fadd2_rn(u, u), w);
-        }
-        DFT<R3, false>::run(v);
+        for (int q = 0; q < R3; ++q) sq[q] = square(v[q]);
+        DFT<R3, false>::run(sq, v);
         ip_store_run<R3>(s4, v, b);
     }
+    static_assert(32 % R3 == 0, "a thread's index within a block's R3 is the same in every round");
+    ip_tw_load<Cat, R2, R3>(w2, p.tw, lane % R3);
     __syncwarp();
 #pragma unroll 1
     for (int t = lane; t < BPW * R3; t += 32) {
@@ -264,6 +264,15 @@ __global__ void __launch_bounds__(CfgI<N>::NTR, CfgI<N>::MBR) k_rows_ip(Pointers
     }
 }
 
+template <int N>
+__global__ void __launch_bounds__(CfgI<N>::NTR, CfgI<N>::MBR) k_rows_ip(Pointers p0)
+{
+    const Pointers p = p0.member(blockIdx.y);
+    using C = CfgI<N>;
+    extern __shared__ __align__(16) float4 s4[];
+    rows_ip<N, C::NTR>(p, blockIdx.x, s4, threadIdx.x);
+}
+
 // ------------------------------------------------------------------------------------------
 // Column pass: column kx: D, E -> z-forward -> FN, Crank-Nicolson / AB2, FNM1 <- FN, velocity
 // recovery -> z-inverse -> U, W.  The column arrives by cp.async in natural order; a thread waits
@@ -271,21 +280,18 @@ __global__ void __launch_bounds__(CfgI<N>::NTR, CfgI<N>::MBR) k_rows_ip(Pointers
 // run along kz, so om2 and fnm1 are read and written coalesced; the 3/2 band's slots are zeros known
 // at compile time where they lie wholly in it.
 // ------------------------------------------------------------------------------------------
-template <int N>
-__global__ void __launch_bounds__(CfgI<N>::NTC, CfgI<N>::MBC) k_cols_ip(Pointers p0, int first, int hist_slot)
+// First half, by NT threads: up to the first stage of the inverse; returns this thread's (E, Z) sums.
+// The threads must pass a barrier before cols_ip_inverse.
+template <int N, int NT>
+__device__ __forceinline__ double2 cols_ip_forward(const Pointers &p, int kx, int first, float4 *s4, int tid)
 {
-    const Pointers p = p0.member(blockIdx.y);
     using C = CfgI<N>;
     using P = typename C::ColPlan;
-    using Cat = IpCat<N>;
-    constexpr int L = C::L, H = C::H, NT = C::NTC, R1 = P::R1, R2 = P::R2, R3 = P::R3, B1 = P::B1;
+    using Cat = TwCat<N>;
+    constexpr int L = C::L, H = C::H, R1 = P::R1, R2 = P::R2, R3 = P::R3, B1 = P::B1;
     constexpr int S3 = R1 * R2, NLO = (H + S3 - 1) / S3, HI0 = (L - H) / S3;
     static_assert(HI0 + NLO == R3 && NLO <= HI0, "retained slots");
     static_assert(B1 % 32 == 0, "whole warps in the first and last stage");
-    extern __shared__ __align__(16) float4 s4[];
-    __shared__ double2 red[NT / 32];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int kx = blockIdx.x;
     float2 *om2c = p.om2 + (size_t)kx * N;
     float2 *fnc = p.fnm1 + (size_t)kx * N;
     static_assert(B1 % widx_rows == 0, "stride");
@@ -305,8 +311,7 @@ __global__ void __launch_bounds__(CfgI<N>::NTC, CfgI<N>::MBC) k_cols_ip(Pointers
         prefetch_l2(om2c + o);
         prefetch_l2(fnc + o);
     }
-    float2 w1[R1], w2[R2];
-    ip_tw_load<Cat, R1, B1>(w1, p.tw, tid < B1 ? tid : 0);
+    float2 w2[R2], w3[R3];
 #pragma unroll 1
     for (int i = 0; i < ND1; ++i) {
         const int j = tid + i * NT;
@@ -319,22 +324,19 @@ __global__ void __launch_bounds__(CfgI<N>::NTC, CfgI<N>::MBC) k_cols_ip(Pointers
             v[r] = {make_float2(x.x, x.z), make_float2(x.y, x.w)};
         }
         DFT<R1, false>::run(v);
-        ip_twiddle<R1, false>(v, w1);
-        if (j + NT < B1) ip_tw_load<Cat, R1, B1>(w1, p.tw, j + NT);
         __syncwarp();  // the swizzled positions are other lanes' inputs
         ip_store<R1, B1>(s4, v, j ^ ((j / R3) & 7));
     }
-    static_assert(32 % R3 == 0, "a thread's index within a block's R3 is the same in every round");
-    ip_tw_load<Cat, R2, R3>(w2, p.tw, lane % R3);
     __syncthreads();
 #pragma unroll 1
     for (int t = tid; t < R1 * R3; t += NT) {
         const int i3 = t % R3, i1 = t / R3;
         const int b = i1 * B1 + (i3 ^ (i1 & 7));
         cpair v[R2];
+        ip_tw_load<Cat, R2, R1>(w2, p.tw, i1);
         ip_load<R2, R3>(v, s4, b);
-        DFT<R2, false>::run(v);
         ip_twiddle<R2, false>(v, w2);
+        DFT<R2, false>::run(v);
         ip_store<R2, R3>(s4, v, b);
     }
     const StepParams prm = *p.prm;
@@ -363,7 +365,9 @@ __global__ void __launch_bounds__(CfgI<N>::NTC, CfgI<N>::MBC) k_cols_ip(Pointers
             }
         }
         cpair v[R3];
+        ip_tw_load<Cat, R3, R1 * R2>(w3, p.tw, j);
         ip_load_run<R3>(v, s4, b);
+        ip_twiddle<R3, false>(v, w3);
         DFT<R3, false>::run(v);
 #pragma unroll
         for (int q = NLO; q < HI0; ++q) czero(v[q]);
@@ -401,12 +405,60 @@ __global__ void __launch_bounds__(CfgI<N>::NTC, CfgI<N>::MBC) k_cols_ip(Pointers
         DFT<R3, true>::run(v);
         ip_store_run<R3>(s4, v, b);
     }
+    return ez;
+}
+
+// Second half: the inverse transform's other stages and the U, W column.
+template <int N, int NT>
+__device__ __forceinline__ void cols_ip_inverse(const Pointers &p, int kx, float4 *s4, int tid)
+{
+    using C = CfgI<N>;
+    using P = typename C::ColPlan;
+    using Cat = TwCat<N>;
+    constexpr int L = C::L, H = C::H, R1 = P::R1, R2 = P::R2, R3 = P::R3, B1 = P::B1;
+    constexpr size_t ZS = (size_t)(B1 / widx_rows) * H * widx_kx_stride;
+    float2 w1[R1], w2[R2];
+    ip_tw_load<Cat, R2, R3>(w2, p.tw, tid % R3);
+#pragma unroll 1
+    for (int t = tid; t < R1 * R3; t += NT) {
+        const int i3 = t % R3, i1 = t / R3;
+        const int b = i1 * B1 + (i3 ^ (i1 & 7));
+        cpair v[R2];
+        ip_load<R2, R3>(v, s4, b);
+        ip_twiddle<R2, true>(v, w2);
+        DFT<R2, true>::run(v);
+        ip_store<R2, R3>(s4, v, b);
+    }
+    ip_tw_load<Cat, R1, B1>(w1, p.tw, tid < B1 ? tid : 0);
+    __syncthreads();
+#pragma unroll 1
+    for (int j = tid; j < B1; j += NT) {
+        cpair v[R1];
+        ip_load<R1, B1>(v, s4, j ^ ((j / R3) & 7));
+        ip_twiddle<R1, true>(v, w1);
+        if (j + NT < B1) ip_tw_load<Cat, R1, B1>(w1, p.tw, j + NT);
+        DFT<R1, true>::run(v);
+        float4 *ptr = reinterpret_cast<float4 *>(p.work + widx<L, H>(0, j, kx));
+#pragma unroll
+        for (int r = 0; r < R1; ++r) ptr[r * (ZS / 2)] = make_float4(v[r].re.x, v[r].im.x, v[r].re.y, v[r].im.y);
+    }
+}
+
+template <int N>
+__global__ void __launch_bounds__(CfgI<N>::NTC, CfgI<N>::MBC) k_cols_ip(Pointers p0, int first, int hist_slot)
+{
+    const Pointers p = p0.member(blockIdx.y);
+    using C = CfgI<N>;
+    constexpr int H = C::H, NT = C::NTC;
+    extern __shared__ __align__(16) float4 s4[];
+    __shared__ double2 red[NT / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, kx = blockIdx.x;
+    double2 ez = cols_ip_forward<N, NT>(p, kx, first, s4, tid);
     for (int o = 16; o > 0; o >>= 1) {
         ez.x += __shfl_xor_sync(0xffffffffu, ez.x, o);
         ez.y += __shfl_xor_sync(0xffffffffu, ez.y, o);
     }
     if (lane == 0) red[warp] = ez;
-    ip_tw_load<Cat, R2, R3>(w2, p.tw, lane % R3);
     __syncthreads();
     // energy / enstrophy: per-column partials, the last column's first warp sums them (deterministic)
     if (warp == 0) {
@@ -440,29 +492,7 @@ __global__ void __launch_bounds__(CfgI<N>::NTC, CfgI<N>::MBC) k_cols_ip(Pointers
             }
         }
     }
-#pragma unroll 1
-    for (int t = tid; t < R1 * R3; t += NT) {
-        const int i3 = t % R3, i1 = t / R3;
-        const int b = i1 * B1 + (i3 ^ (i1 & 7));
-        cpair v[R2];
-        ip_load<R2, R3>(v, s4, b);
-        ip_twiddle<R2, true>(v, w2);
-        DFT<R2, true>::run(v);
-        ip_store<R2, R3>(s4, v, b);
-    }
-    ip_tw_load<Cat, R1, B1>(w1, p.tw, tid < B1 ? tid : 0);
-    __syncthreads();
-#pragma unroll 1
-    for (int j = tid; j < B1; j += NT) {
-        cpair v[R1];
-        ip_load<R1, B1>(v, s4, j ^ ((j / R3) & 7));
-        ip_twiddle<R1, true>(v, w1);
-        if (j + NT < B1) ip_tw_load<Cat, R1, B1>(w1, p.tw, j + NT);
-        DFT<R1, true>::run(v);
-        float4 *ptr = reinterpret_cast<float4 *>(p.work + widx<L, H>(0, j, kx));
-#pragma unroll
-        for (int r = 0; r < R1; ++r) ptr[r * (ZS / 2)] = make_float4(v[r].re.x, v[r].im.x, v[r].re.y, v[r].im.y);
-    }
+    cols_ip_inverse<N, NT>(p, kx, s4, tid);
 }
 
 }  // namespace dns2d

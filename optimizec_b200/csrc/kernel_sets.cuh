@@ -172,19 +172,13 @@ struct LaunchC {
     using C = CfgC<N>;
     static constexpr size_t sm1 = (size_t)C::MP * sizeof(float2);
     static constexpr size_t sm2 = 2 * sm1;
-    static constexpr size_t smI = (size_t)C::L * 2 * sizeof(float2);  // the in-place passes' two arrays
 
     static cudaError_t setup()
     {
         const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
         cudaError_t e;
-        if constexpr (CfgI<N>::enabled) {
-            if ((e = cudaFuncSetAttribute(k_rows_ip<N>, a, (int)smI)) != cudaSuccess) return e;
-            if ((e = cudaFuncSetAttribute(k_cols_ip<N>, a, (int)smI)) != cudaSuccess) return e;
-        } else {
-            if ((e = cudaFuncSetAttribute(k_rows_step_c<N>, a, (int)sm1)) != cudaSuccess) return e;
-            if ((e = cudaFuncSetAttribute(k_cols_step_c<N>, a, (int)sm2)) != cudaSuccess) return e;
-        }
+        if ((e = cudaFuncSetAttribute(k_rows_step_c<N>, a, (int)sm1)) != cudaSuccess) return e;
+        if ((e = cudaFuncSetAttribute(k_cols_step_c<N>, a, (int)sm2)) != cudaSuccess) return e;
         if ((e = cudaFuncSetAttribute(k_cols_init_c<N>, a, (int)sm2)) != cudaSuccess) return e;
         if ((e = cudaFuncSetAttribute(k_rows_velocity_c<N>, a, (int)sm1)) != cudaSuccess) return e;
         if ((e = cudaFuncSetAttribute(k_rows_from_phys_c<N>, a, (int)sm1)) != cudaSuccess) return e;
@@ -194,13 +188,11 @@ struct LaunchC {
     }
     static void rows_step(const Pointers &p, cudaStream_t s, int ny)
     {
-        if constexpr (CfgI<N>::enabled) k_rows_ip<N><<<dim3(C::L / 2, ny), CfgI<N>::NTR, smI, s>>>(p);
-        else k_rows_step_c<N><<<dim3(4 * C::L, ny), C::NT, sm1, s>>>(p);
+        k_rows_step_c<N><<<dim3(4 * C::L, ny), C::NT, sm1, s>>>(p);
     }
     static void cols_step(const Pointers &p, int first, int slot, cudaStream_t s, int ny)
     {
-        if constexpr (CfgI<N>::enabled) k_cols_ip<N><<<dim3(C::H, ny), CfgI<N>::NTC, smI, s>>>(p, first, slot);
-        else k_cols_step_c<N><<<dim3(4 * C::H, ny), C::NT, sm2, s>>>(p, first, slot);
+        k_cols_step_c<N><<<dim3(4 * C::H, ny), C::NT, sm2, s>>>(p, first, slot);
     }
     static void cols_init(const Pointers &p, const float2 *uw, int mode, cudaStream_t s, int ny)
     {
