@@ -26,14 +26,14 @@
 // and 4096 have the auto-sort kernels' results bit for bit.  It matters: FP32 rounding of the products, times
 // k^2, is 1e-3 of the field's RMS in single modes of the corners, and a run compared with an earlier one
 // would show it.  A first transform by decimation in frequency (twiddles after a butterfly, fetched once)
-// was 1-9 % faster (N = 4096 386 us per step, 2048 89.7; here 392, 98), N = 8192 / 9216 on three-stage in-place
+// was 1-9 % faster (N = 4096 386 us per step, 2048 89.7; with decimation in time 392, 98), N = 8192 / 9216 on three-stage in-place
 // passes twice as fast as the clusters (1.75 / 2.55 ms), N = 512 and 256 15.3 and 10.6 us (20.6 and 12.1) and the
 // 64-member ensemble 77 us per step (125): all with other rounding, further from an earlier run than two runs may be.
 //
 // Bounds (N = 4096 on B200, 1965 MHz; ncu): the row pass is bound by the L1 / shared-memory data
 // pipe (67-75 % of its cycles busy; 24 % before the loads' and twiddles' share fell), the column pass
 // by the latency of its phases at two CTAs per SM (HBM 35 %, issue 32 %).  Measured (rows / columns,
-// one launch): N = 4096 0.254 / 0.293 -> 0.193 / 0.211 ms, N = 2048 67.6 / 71.7 -> 52.1 / 58.6 us,
+// one launch): N = 4096 0.254 / 0.293 -> 0.193 / 0.201 ms, N = 2048 67.6 / 71.7 -> 52.1 / 54.7 us,
 // N = 1024 27.0 / 28.2 -> 20.3 / 23.2 us against the auto-sort kernels that these replace (one row,
 // or one array and thread group, per 384 threads).
 // Tried and slower, or no faster: each sequence on its own lane with scalar butterflies (rows 0.185,
@@ -273,6 +273,34 @@ __global__ void __launch_bounds__(CfgI<N>::NTR, CfgI<N>::MBR) k_rows_ip(Pointers
     rows_ip<N, C::NTR>(p, blockIdx.x, s4, threadIdx.x);
 }
 
+// The factors of cn_update and recover_velocity for one mode, in FP64 and each rounded once to float as
+// there, from one reciprocal in place of two divisions: r = 1 / (K^2 (1 + a)), 1 / (1 + a) = r K^2,
+// 1 / K^2 = r (1 + a).  The reciprocal is the PTX instruction's approximation (relative error 2^-20) and two
+// steps of Newton's iteration x <- x + x (1 - d x), which squares the error each time.  The column pass
+// waits for the chains of these (N = 4096 on B200: columns 211 -> 201 us; 2048 58.6 -> 54.7).
+struct ModeFactors {
+    float d1, c2, c3, gu, gw;
+    double invK2;  // 0 at K = 0
+};
+__device__ __forceinline__ ModeFactors mode_factors(int kx, int kz, double hvdt, double c2n, double c3n)
+{
+    const int k2 = kx * kx + kz * kz;
+    const double K2 = (double)k2, a = hvdt * K2, q = 1.0 + a, s = k2 ? K2 : 1.0, d = s * q;
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+    r = fma(r, fma(-d, r, 1.0), r);
+    r = fma(r, fma(-d, r, 1.0), r);
+    const double inv = r * s, invK2 = k2 ? r * q : 0.0;
+    ModeFactors f;
+    f.d1 = (float)(-2.0 * a * inv);
+    f.c2 = (float)(c2n * inv);
+    f.c3 = (float)(c3n * inv);
+    f.gu = (float)((double)kz * invK2);
+    f.gw = (float)((double)kx * invK2);
+    f.invK2 = invK2;
+    return f;
+}
+
 // ------------------------------------------------------------------------------------------
 // Column pass: column kx: D, E -> z-forward -> FN, Crank-Nicolson / AB2, FNM1 <- FN, velocity
 // recovery -> z-inverse -> U, W.  The column arrives by cp.async in natural order; a thread waits
@@ -347,7 +375,6 @@ __device__ __forceinline__ double2 cols_ip_forward(const Pointers &p, int kx, in
     const double c3n = -0.5 * (double)dt * (double)cnm1;
     const float divxz = (float)(1.0 / ((double)L * (double)L));
     double2 ez = make_double2(0.0, 0.0);
-    const double wgt = (kx == 0) ? 0.5 : 1.0;
     __syncthreads();
 #pragma unroll 1
     for (int j = tid; j < S3; j += NT) {
@@ -388,24 +415,24 @@ __device__ __forceinline__ double2 cols_ip_forward(const Pointers &p, int kx, in
                     fn.y = (ga * d.y + g2a2 * e.y) * divxz;
                     if (p.force) fn = add_forcing(fn, p, kx, iz, N);
                 }
-                const double K2 = (double)kx * kx + (double)kz * kz;
-                const float2 on = cn_update(om[q], fn, fo[q], K2, hvdt, c2n, c3n);
+                const ModeFactors f = mode_factors(kx, kz, hvdt, c2n, c3n);
+                const float2 on = make_float2(om[q].x + fmaf(f.d1, om[q].x, fmaf(f.c2, fn.x, f.c3 * fo[q].x)),
+                                              om[q].y + fmaf(f.d1, om[q].y, fmaf(f.c2, fn.y, f.c3 * fo[q].y)));
                 om2c[iz] = on;
                 fnc[iz] = fn;
-                double invK2;
-                float2 u, w;
-                recover_velocity(kx, kz, on, u, w, invK2);
-                uw = {make_float2(u.x, w.x), make_float2(u.y, w.y)};
+                // u = -i gu om, w = i gw om
+                uw = {make_float2(f.gu * on.y, -f.gw * on.y), make_float2(-f.gu * on.x, f.gw * on.x)};
                 const double pw = (double)on.x * on.x + (double)on.y * on.y;
-                ez.x += wgt * pw * invK2;
-                ez.y += wgt * pw;
+                ez.x = fma(pw, f.invK2, ez.x);
+                ez.y += pw;
             }
             v[slot] = uw;
         }
         DFT<R3, true>::run(v);
         ip_store_run<R3>(s4, v, b);
     }
-    return ez;
+    const double wgt = (kx == 0) ? 0.5 : 1.0;  // 1/2 * (1 on kx = 0, else 2)
+    return make_double2(ez.x * wgt, ez.y * wgt);
 }
 
 // Second half: the inverse transform's other stages and the U, W column.
