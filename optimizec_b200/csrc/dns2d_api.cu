@@ -1971,6 +1971,11 @@ struct dns2d_batch {
     int stall_member = -1;
     int ens_grid = 0;
     int tiles_per_item = 8, groups_per_item = 4;  // persistent launch work-item size (powers of two)
+    // the [iz][ix] copy of a member's field on its way to the host, as large as the largest member's:
+    // allocated by the first read, kept (an allocation and a release per read took 0.5 ms of a 64-member
+    // ensemble's reads each); the lock keeps one read's transpose and copy together on the stream
+    float2 *out_stage = nullptr;
+    std::mutex out_lock;
     bool initialised = false;
     std::string err;
 };
@@ -1999,6 +2004,7 @@ int bfail(dns2d_batch *b, int code, const char *what, cudaError_t e = cudaSucces
 extern "C" void dns2d_batch_destroy(dns2d_batch *b)
 {
     if (!b) return;
+    if (b->out_stage) cudaFreeAsync(b->out_stage, b->stream);
     if (b->stream) cudaStreamSynchronize(b->stream);
     for (auto &kv : b->graphs) cudaGraphExecDestroy(kv.second);
     for (BatchGroup &g : b->groups) {
@@ -2474,13 +2480,18 @@ extern "C" int dns2d_batch_get_om2(dns2d_batch *b, int member, float *om2)
     const auto [gi, k] = b->where[(size_t)member];
     BatchGroup &g = b->groups[(size_t)gi];
     const size_t nom = (size_t)g.N * g.H;
-    float2 *stage = nullptr;
-    BATCH_CUDA(cudaMallocAsync((void **)&stage, nom * 8, b->stream), "staging");
-    dim3 tb(32, 8), tg((g.N + 31) / 32, (g.H + 31) / 32);
-    k_transpose_c64<<<tg, tb, 0, b->stream>>>(g.om2 + (size_t)k * nom, stage, g.H, g.N);
-    BATCH_CUDA(cudaGetLastError(), "transpose");
-    BATCH_CUDA(cudaMemcpyAsync(om2, stage, nom * 8, cudaMemcpyDeviceToHost, b->stream), "om2 copy");
-    BATCH_CUDA(cudaFreeAsync(stage, b->stream), "staging free");
+    {
+        std::lock_guard<std::mutex> lock(b->out_lock);
+        if (!b->out_stage) {
+            size_t most = 0;
+            for (const BatchGroup &q : b->groups) most = std::max(most, (size_t)q.N * q.H);
+            BATCH_CUDA(cudaMallocAsync((void **)&b->out_stage, most * 8, b->stream), "staging");
+        }
+        dim3 tb(32, 8), tg((g.N + 31) / 32, (g.H + 31) / 32);
+        k_transpose_c64<<<tg, tb, 0, b->stream>>>(g.om2 + (size_t)k * nom, b->out_stage, g.H, g.N);
+        BATCH_CUDA(cudaGetLastError(), "transpose");
+        BATCH_CUDA(cudaMemcpyAsync(om2, b->out_stage, nom * 8, cudaMemcpyDeviceToHost, b->stream), "om2 copy");
+    }
     BATCH_CUDA(cudaStreamSynchronize(b->stream), "om2 sync");
     return DNS2D_OK;
 }
