@@ -586,10 +586,23 @@ cudaError_t grow(void **p, size_t *cap, size_t need, size_t elem)
     return e;
 }
 
+// dynamic shared memory of k_gemm_rows for KS K steps, and of k_gemm_splitk for MT M tiles
+constexpr size_t rows_smem(int KS)
+{
+    return 1024 + (size_t)(KS * B_BLOCK * 2 + 1023) / 1024 * 1024 + (size_t)kRowStages * KS * A_BLOCK * 2;
+}
+constexpr size_t splitk_smem(int MT) { return 1024 + (size_t)kSplitStages * KC * (MT * A_BLOCK + B_BLOCK) * 2; }
+static_assert(rows_smem(MAX_KS) <= 227 * 1024 && splitk_smem(MAX_MT) <= 227 * 1024, "shared memory of a CTA");
+
 cudaError_t ensure(Work &wk, size_t a_el, size_t b_el, size_t part_f, cudaStream_t st)
 {
     cudaError_t e;
     if (!wk.err) {
+        // the limit belongs to the function: the most that any layer of any network asks for, so that networks
+        // on several host threads set the same value
+        const cudaFuncAttribute sm = cudaFuncAttributeMaxDynamicSharedMemorySize;
+        if ((e = cudaFuncSetAttribute(k_gemm_rows, sm, (int)rows_smem(MAX_KS))) != cudaSuccess) return e;
+        if ((e = cudaFuncSetAttribute(k_gemm_splitk, sm, (int)splitk_smem(MAX_MT))) != cudaSuccess) return e;
         if ((e = cudaMalloc((void **)&wk.err, 4)) != cudaSuccess) return e;
         if ((e = cudaMemsetAsync(wk.err, 0, 4, st)) != cudaSuccess) return e;
     }
@@ -620,10 +633,7 @@ cudaError_t run_rows(GemmArgs g, Work &wk, cudaStream_t st)
     g.A = wk.A;
     g.Bm = wk.Bm;
     g.err = wk.err;
-    const size_t smem = 1024 + (size_t)(g.KS * B_BLOCK * 2 + 1023) / 1024 * 1024 + (size_t)kRowStages * g.KS * A_BLOCK * 2;
-    cudaError_t e = cudaFuncSetAttribute(k_gemm_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    k_gemm_rows<<<std::min(g.MT, sm_count()), kRowThreads, smem, st>>>(g);
+    k_gemm_rows<<<std::min(g.MT, sm_count()), kRowThreads, rows_smem(g.KS), st>>>(g);
     return cudaGetLastError();
 }
 
@@ -694,10 +704,7 @@ cudaError_t conv_wgrad(const float *x, int Ci, const float *dz, int Co, float *d
     g.KS = KS;
     g.part = wk.part;
     g.err = wk.err;
-    const size_t smem = 1024 + (size_t)kSplitStages * KC * (MT * A_BLOCK + B_BLOCK) * 2;
-    if ((e = cudaFuncSetAttribute(k_gemm_splitk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
-        return e;
-    k_gemm_splitk<<<G, kGemmThreads, smem, st>>>(g);
+    k_gemm_splitk<<<G, kGemmThreads, splitk_smem(MT), st>>>(g);
     k_reduce_wgrad<<<blocks_for((long long)Co * Ci * 9 + Co), 256, 0, st>>>(wk.part, G, MT, Ci, Co, dw, db);
     return cudaGetLastError();
 }

@@ -331,17 +331,24 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_cnn_net(const __grid_constan
 
 }  // namespace
 
-int net_stages_that_fit(int L)
+// most dynamic shared memory that a CTA of k_cnn_net can have (0: unknown)
+static size_t net_smem_limit()
 {
-    if (L < 3 || L > kNetMaxLayers) return 0;
     int dev = 0, optin = 0;
     cudaFuncAttributes fa{};
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
         cudaFuncGetAttributes(&fa, k_cnn_net) != cudaSuccess)
         return 0;
+    return (size_t)optin - fa.sharedSizeBytes;
+}
+
+int net_stages_that_fit(int L)
+{
+    if (L < 3 || L > kNetMaxLayers) return 0;
+    const size_t limit = net_smem_limit();
     for (int s = kNetMaxStages; s >= 2; --s)
-        if (net_smem_bytes(L, s) + fa.sharedSizeBytes <= (size_t)optin) return s;
+        if (net_smem_bytes(L, s) <= limit) return s;
     return 0;
 }
 
@@ -352,7 +359,10 @@ cudaError_t net_launch(const NetLaunch &q_in, cudaStream_t stream, int *grid_out
     NetLaunch q = q_in;
     cudaError_t e;
     const size_t smem = net_smem_bytes(q.L, q.stages);
-    if ((e = cudaFuncSetAttribute(k_cnn_net, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
+    // the limit belongs to the function: the same for networks of every depth, on any host thread
+    const size_t limit = net_smem_limit();
+    if (smem > limit) return cudaErrorInvalidConfiguration;
+    if ((e = cudaFuncSetAttribute(k_cnn_net, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit)) != cudaSuccess)
         return e;
     int dev = 0, sms = 0, per_sm = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;

@@ -520,12 +520,22 @@ uint4 *input_planes(const Net &n, const Planes &p, int l)
     return p.act + off;
 }
 
-size_t wgrad_smem(int rows, int nchi, int ncho)
+// dynamic shared memory of k_conv_planes for Cin input channels, and of k_wgrad_planes
+constexpr size_t conv_smem(int Cin)
+{
+    return (size_t)ksteps_of(Cin) * 1024 + (size_t)kConvStages * (point_of(Cin) ? 1 : 3) * planes_of(Cin) * kSeg;
+}
+constexpr size_t wgrad_smem(int rows, int nchi, int ncho)
 {
     // the last stage's M tile reaches 16 planes from its start
-    const int planes = wgrad_planes(rows, nchi, ncho), tail = std::max(16 - planes, 0);
+    const int planes = wgrad_planes(rows, nchi, ncho), tail = planes < 16 ? 16 - planes : 0;
     return (size_t)(kWgradStages * planes + tail) * kPlane;
 }
+constexpr int kMaxC = 32;  // of supported()
+static_assert(conv_smem(kMaxC) >= conv_smem(16) && conv_smem(kMaxC) >= conv_smem(3) && conv_smem(kMaxC) >= conv_smem(1) &&
+                  wgrad_smem(3, 4, 4) >= wgrad_smem(3, 2, 2) && wgrad_smem(3, 4, 4) >= wgrad_smem(1, 4, 4) &&
+                  wgrad_smem(3, 4, 4) <= 227 * 1024,
+              "the most shared memory that any layer asks for");
 
 cudaError_t conv(const Net &n, ConvArgs a, int Cin, cudaStream_t st)
 {
@@ -537,10 +547,7 @@ cudaError_t conv(const Net &n, ConvArgs a, int Cin, cudaStream_t st)
     a.W = n.W;
     a.tiles_img = (n.H * (n.W + 2) + 127) / 128;
     a.tiles = a.tiles_img * n.B;
-    const size_t smem = (size_t)a.KS * 1024 + (size_t)kConvStages * a.rows * a.nch * kSeg;
-    cudaError_t e = cudaFuncSetAttribute(k_conv_planes, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    k_conv_planes<<<std::min(a.tiles, kConvCtas * sm_count()), kConvThreads, smem, st>>>(a);
+    k_conv_planes<<<std::min(a.tiles, kConvCtas * sm_count()), kConvThreads, conv_smem(Cin), st>>>(a);
     return cudaGetLastError();
 }
 
@@ -559,10 +566,7 @@ cudaError_t wgrad(const Net &n, const uint4 *x, const uint4 *dz, int l, Planes &
     a.part = p.part;
     a.err = p.err;
     const int G = std::min(a.items, sm_count());
-    const size_t smem = wgrad_smem(a.rows, a.nchi, a.ncho);
-    cudaError_t e = cudaFuncSetAttribute(k_wgrad_planes, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    k_wgrad_planes<<<G, kWgradThreads, smem, st>>>(a);
+    k_wgrad_planes<<<G, kWgradThreads, wgrad_smem(a.rows, a.nchi, a.ncho), st>>>(a);
     float *dw = n.grad + n.woff[l], *db = dw + (size_t)n.co[l] * n.ci[l] * 9;
     // a point tensor's centre tap is the tensor itself
     k_reduce_planes<<<dim3(8 * a.rows * a.nchi + 1, a.rows), 256, 0, st>>>(
@@ -585,6 +589,11 @@ cudaError_t reserve(const Net &n, Planes &p, cudaStream_t st)
     }
     cudaError_t e;
     if (!p.err) {
+        // the limit belongs to the function: the most that any layer of any network asks for, so that networks
+        // on several host threads set the same value
+        const cudaFuncAttribute sm = cudaFuncAttributeMaxDynamicSharedMemorySize;
+        if ((e = cudaFuncSetAttribute(k_conv_planes, sm, (int)conv_smem(kMaxC))) != cudaSuccess) return e;
+        if ((e = cudaFuncSetAttribute(k_wgrad_planes, sm, (int)wgrad_smem(3, 4, 4))) != cudaSuccess) return e;
         if ((e = cudaMalloc((void **)&p.err, 4)) != cudaSuccess) return e;
         if ((e = cudaMemsetAsync(p.err, 0, 4, st)) != cudaSuccess) return e;
     }
