@@ -639,6 +639,12 @@ cudaError_t run_rows(GemmArgs g, Work &wk, cudaStream_t st)
 
 }  // namespace
 
+cudaError_t reserve_fwd(int C, int B, int H, int W, Work &wk, cudaStream_t st)
+{
+    const int MT = (B * H * W + BM - 1) / BM, KS = ksteps_of(C);
+    return ensure(wk, (size_t)MT * KS * A_BLOCK, (size_t)KS * B_BLOCK, 0, st);
+}
+
 cudaError_t conv_fwd(const float *x, int Ci, const float *w, const float *bias, int Co, float *z, float *a, int B,
                      int H, int W, Work &wk, cudaStream_t st)
 {

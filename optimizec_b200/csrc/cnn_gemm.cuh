@@ -64,6 +64,8 @@ cudaError_t conv_dgrad(const float *dz, int Co, const float *w, int Ci, const fl
 // dw[co][ci][tap] = sum dz[b][co][p] x[b][ci][p + tap], db[co] = sum dz[b][co][p]
 cudaError_t conv_wgrad(const float *x, int Ci, const float *dz, int Co, float *dw, float *db, int B, int H, int W,
                        Work &wk, cudaStream_t st);
+// the buffers of conv_fwd for layers of up to C channels, so that it can be captured
+cudaError_t reserve_fwd(int C, int B, int H, int W, Work &wk, cudaStream_t st);
 void work_free(Work &wk);
 
 }  // namespace cnngemm

@@ -3355,8 +3355,20 @@ static int closure_device_step(dns2d_state *s, int first, int slot)
     return DNS2D_OK;
 }
 
+// buffers of the attached network that a closed step would otherwise have to grow while it is captured: in
+// training mode a closed step runs the network as im2col GEMMs, training itself need not (cnn_train.cuh)
+static int closure_buffers(dns2d_state *s)
+{
+    dns2d_cnn *n = s->cnn;
+    if (!n->train_tc || (s->closure_tc && cnn_tc_supported(n, s->L, s->L))) return DNS2D_OK;
+    DNS2D_CUDA(dns2d::cnngemm::reserve_fwd(std::max(n->channels, 3), 1, s->L, s->L, n->gw, s->stream),
+               "closure network buffers");
+    return DNS2D_OK;
+}
+
 static int closure_run(dns2d_state *s, int nsteps, double *E_hist, double *Z_hist)
 {
+    if (const int rc = closure_buffers(s)) return rc;
     const size_t nom = (size_t)s->N * s->H, nwork = 2 * (size_t)s->L * s->H;
     if (s->closure_check != 2) {
         // device-side energy gate; chunks of up to 128 closed steps are captured CUDA graphs
