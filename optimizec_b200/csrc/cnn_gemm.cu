@@ -606,8 +606,10 @@ cudaError_t ensure(Work &wk, size_t a_el, size_t b_el, size_t part_f, cudaStream
         if ((e = cudaMalloc((void **)&wk.err, 4)) != cudaSuccess) return e;
         if ((e = cudaMemsetAsync(wk.err, 0, 4, st)) != cudaSuccess) return e;
     }
-    if (a_el > wk.A_cap || b_el > wk.B_cap || part_f > wk.part_cap)
+    if (a_el > wk.A_cap || b_el > wk.B_cap || part_f > wk.part_cap) {
         if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;  // the old buffers may be in use
+        wk.gen += 1;
+    }
     if ((e = grow((void **)&wk.A, &wk.A_cap, a_el, 2)) != cudaSuccess) return e;
     if ((e = grow((void **)&wk.Bm, &wk.B_cap, b_el, 2)) != cudaSuccess) return e;
     return grow((void **)&wk.part, &wk.part_cap, part_f, 4);

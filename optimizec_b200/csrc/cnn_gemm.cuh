@@ -53,6 +53,7 @@ struct Work {
     float *part = nullptr;
     size_t part_cap = 0;          // floats
     int *err = nullptr;           // 1: an mbarrier wait ran out
+    long long gen = 0;            // counts replaced buffers
 };
 
 // z = conv(x) + bias and, when a is set, a = GELU(z); x [B][Ci][H][W], z / a [B][Co][H][W]

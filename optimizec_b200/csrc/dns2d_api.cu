@@ -392,6 +392,7 @@ struct dns2d_state {
     unsigned int *gate_counter = nullptr;
     unsigned long long *gate_off = nullptr; // device count of gated-off steps
     std::map<int, cudaGraphExec_t> closure_graphs;
+    long long closure_buf_gen = -1;  // of the network's buffers that those graphs refer to
     float *closure_in = nullptr;
     long long closure_steps = 0, closure_fallbacks = 0;
     double closure_E = -1.0;
@@ -2621,6 +2622,7 @@ struct dns2d_cnn {
     float *wpack = nullptr;        // packed weights of the FP32 convolutions, per layer forward and data gradient
     std::vector<size_t> pk_fwd, pk_bwd;
     size_t cap_elems = 0;          // per activation tensor: B * max(C, 3) * H * W
+    long long buf_gen = 0;         // counts replaced buffers that a captured closed step refers to
     int capB = 0, capH = 0, capW = 0;
     double *part = nullptr;
     long long step = 0;
@@ -2675,6 +2677,8 @@ uint64_t sm64(uint64_t &s)
 int cnn_reserve(dns2d_cnn *n, int B, int H, int W)
 {
     if (B <= n->capB && H == n->capH && W == n->capW) return DNS2D_OK;
+    n->buf_gen += 1;
+    n->capB = 0;
     CNN_CUDA(cudaStreamSynchronize(n->stream), "sync");
     for (float *p : n->z) cudaFree(p);
     for (float *p : n->a) cudaFree(p);
@@ -2826,6 +2830,8 @@ int cnn_tc_reserve(dns2d_cnn *n, int B, int H, int W)
         cudaFree(n->act_tc[0]);
         cudaFree(n->act_tc[1]);
         n->act_tc[0] = n->act_tc[1] = nullptr;
+        n->act_tc_cap = 0;
+        n->buf_gen += 1;
         CNN_CUDA(cudaMalloc((void **)&n->act_tc[0], need), "tc activation alloc");
         CNN_CUDA(cudaMalloc((void **)&n->act_tc[1], need), "tc activation alloc");
         n->act_tc_cap = need;
@@ -2836,6 +2842,8 @@ int cnn_tc_reserve(dns2d_cnn *n, int B, int H, int W)
         CNN_CUDA(cudaStreamSynchronize(n->stream), "sync");
         cudaFree(n->net_sync);
         n->net_sync = nullptr;
+        n->net_sync_cap = 0;
+        n->buf_gen += 1;
         CNN_CUDA(cudaMalloc((void **)&n->net_sync, words * 4), "network counters alloc");
         CNN_CUDA(cudaMemset(n->net_sync, 0, words * 4), "network counters clear");
         n->net_sync_cap = words;
@@ -2892,6 +2900,8 @@ int cnn_forward_tc_dev(dns2d_cnn *n, int B, int H, int W, const dns2d::cnntc::Fi
                 CNN_CUDA(cudaStreamSynchronize(st), "sync");
                 cudaFree(n->trace);
                 n->trace = nullptr;
+                n->trace_cap = 0;
+                n->buf_gen += 1;
                 CNN_CUDA(cudaMalloc((void **)&n->trace, tiles * kNetTraceSlots * sizeof(unsigned long long)),
                          "trace alloc");
                 n->trace_cap = tiles;
@@ -3355,14 +3365,24 @@ static int closure_device_step(dns2d_state *s, int first, int slot)
     return DNS2D_OK;
 }
 
-// buffers of the attached network that a closed step would otherwise have to grow while it is captured: in
-// training mode a closed step runs the network as im2col GEMMs, training itself need not (cnn_train.cuh)
+// The attached network's buffers for one L x L image, before a closed step is launched or captured: other
+// calls on the network (another image size, a larger batch, training) may have replaced or outgrown
+// those that the closure was attached with, and captured steps refer to them.  In training mode a closed
+// step runs the network as im2col GEMMs, whose buffers training itself need not have (cnn_train.cuh).
 static int closure_buffers(dns2d_state *s)
 {
     dns2d_cnn *n = s->cnn;
-    if (!n->train_tc || (s->closure_tc && cnn_tc_supported(n, s->L, s->L))) return DNS2D_OK;
-    DNS2D_CUDA(dns2d::cnngemm::reserve_fwd(std::max(n->channels, 3), 1, s->L, s->L, n->gw, s->stream),
-               "closure network buffers");
+    const bool tc = cnn_tc_supported(n, s->L, s->L);
+    if (n->train_tc && !(s->closure_tc && tc))
+        DNS2D_CUDA(dns2d::cnngemm::reserve_fwd(std::max(n->channels, 3), 1, s->L, s->L, n->gw, s->stream),
+                   "closure network buffers");
+    if (s->closure_buf_gen == n->buf_gen + n->gw.gen) return DNS2D_OK;
+    int rc = cnn_reserve(n, 1, s->L, s->L);
+    if (!rc && tc) rc = cnn_tc_reserve(n, 1, s->L, s->L);
+    if (rc) return fail(s, rc, "closure network: %s", n->err.c_str());
+    for (auto &kv : s->closure_graphs) cudaGraphExecDestroy(kv.second);
+    s->closure_graphs.clear();
+    s->closure_buf_gen = n->buf_gen + n->gw.gen;
     return DNS2D_OK;
 }
 
@@ -3505,6 +3525,7 @@ extern "C" int dns2d_closure_attach(dns2d_state *s, dns2d_cnn *n, const float *s
     DNS2D_CUDA(cudaMemsetAsync(s->gate_off, 0, 8, s->stream), "gate counter");
     for (auto &kv : s->closure_graphs) cudaGraphExecDestroy(kv.second);
     s->closure_graphs.clear();
+    s->closure_buf_gen = -1;
     int rc = cnn_reserve(n, 1, s->L, s->L);
     if (!rc && cnn_tc_supported(n, s->L, s->L)) {
         rc = cnn_tc_reserve(n, 1, s->L, s->L);
@@ -3550,7 +3571,8 @@ extern "C" int dns2d_closure_forcing(dns2d_state *s, float *force)
     if (!s || !force) return DNS2D_ERR_ARG;
     if (!s->cnn) return fail(s, DNS2D_ERR_STATE, "no closure attached");
     if (!s->initialised) return fail(s, DNS2D_ERR_STATE, "no initial condition");
-    int rc = closure_forcing(s);
+    int rc = closure_buffers(s);
+    if (!rc) rc = closure_forcing(s);
     if (rc) return rc;
     return download_compact(s, s->force, force);
 }
