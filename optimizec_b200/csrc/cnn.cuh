@@ -361,10 +361,15 @@ __global__ void k_mse(const float *__restrict__ pred, const float *__restrict__ 
     if (threadIdx.x == 0) part[blockIdx.x] = red[0];
 }
 
-// Adam (bias-corrected) on the flat parameter vector
+// Adam (bias-corrected) on the flat parameter vector.  With tensor-core training e0 / e1 (nullable) are the wait
+// flags of its kernels: a gradient from a pass in which a wait ran out is not applied, and *steps counts
+// the iterations that were.
 __global__ void k_adam(float *__restrict__ p, const float *__restrict__ g, float *__restrict__ m, float *__restrict__ v,
-                       int n, float lr, float b1, float b2, float eps, float c1, float c2)
+                       int n, float lr, float b1, float b2, float eps, float c1, float c2, const int *e0,
+                       const int *e1, int *steps)
 {
+    if ((e0 && *e0) || (e1 && *e1)) return;
+    if (steps && blockIdx.x == 0 && threadIdx.x == 0) *steps += 1;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float gi = g[i];
         const float mi = b1 * m[i] + (1.0f - b1) * gi;

@@ -2626,6 +2626,7 @@ struct dns2d_cnn {
     int capB = 0, capH = 0, capW = 0;
     double *part = nullptr;
     long long step = 0;
+    int *adam_steps = nullptr;     // iterations that the current dns2d_cnn_train has applied
     float *data_x = nullptr, *data_t = nullptr;  // device-resident training set
     int data_n = 0, data_H = 0, data_W = 0;
     // BF16 tensor-core inference path (cnn_tc.cuh, cnn_net.cuh): packed weights, padded
@@ -3006,6 +3007,7 @@ extern "C" void dns2d_cnn_destroy(dns2d_cnn *n)
     cudaFree(n->gout);
     cudaFree(n->gtmp);
     cudaFree(n->part);
+    cudaFree(n->adam_steps);
     cudaFree(n->data_x);
     cudaFree(n->data_t);
     cudaFree(n->wtc);
@@ -3068,7 +3070,8 @@ extern "C" int dns2d_cnn_create(dns2d_cnn **out, int layers, int channels, uint6
     if (cudaMalloc((void **)&n->params, off * 4) != cudaSuccess || cudaMalloc((void **)&n->grad, off * 4) != cudaSuccess ||
         cudaMalloc((void **)&n->adam_m, off * 4) != cudaSuccess || cudaMalloc((void **)&n->adam_v, off * 4) != cudaSuccess ||
         cudaMalloc((void **)&n->wg_part, std::max(wg, (size_t)148 * dns2d::cnn::kWgCtas * dns2d::cnn::kWgPart) * 4) != cudaSuccess ||
-        cudaMalloc((void **)&n->wpack, pk * 4) != cudaSuccess || cudaMalloc((void **)&n->part, 256 * 8) != cudaSuccess)
+        cudaMalloc((void **)&n->wpack, pk * 4) != cudaSuccess || cudaMalloc((void **)&n->part, 256 * 8) != cudaSuccess ||
+        cudaMalloc((void **)&n->adam_steps, sizeof(int)) != cudaSuccess)
         return bail(DNS2D_ERR_NOMEM);
     if (cudaMemcpy(n->params, p.data(), off * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemset(n->adam_m, 0, off * 4) != cudaSuccess || cudaMemset(n->adam_v, 0, off * 4) != cudaSuccess)
@@ -3101,6 +3104,22 @@ extern "C" int dns2d_cnn_set_params(dns2d_cnn *n, const float *p)
     return DNS2D_OK;
 }
 
+// the tensor-core training GEMMs' wait flags (0 when no GEMM ran), cleared once reported; the stream is
+// synchronised
+static int train_tc_status(dns2d_cnn *n)
+{
+    int flag[2] = {0, 0};
+    if (n->gw.err) CNN_CUDA(cudaMemcpyAsync(flag, n->gw.err, 4, cudaMemcpyDeviceToHost, n->stream), "flag copy");
+    if (n->planes.err)
+        CNN_CUDA(cudaMemcpyAsync(flag + 1, n->planes.err, 4, cudaMemcpyDeviceToHost, n->stream), "flag copy");
+    CNN_CUDA(cudaStreamSynchronize(n->stream), "flag sync");
+    if (!flag[0] && !flag[1]) return DNS2D_OK;
+    if (flag[0]) CNN_CUDA(cudaMemsetAsync(n->gw.err, 0, 4, n->stream), "flag clear");
+    if (flag[1]) CNN_CUDA(cudaMemsetAsync(n->planes.err, 0, 4, n->stream), "flag clear");
+    CNN_CUDA(cudaStreamSynchronize(n->stream), "flag sync");
+    return nfail(n, DNS2D_ERR_TIMEOUT, "tensor-core training GEMM wait timed out");
+}
+
 extern "C" int dns2d_cnn_forward(dns2d_cnn *n, const float *x, int B, int H, int W, float *y)
 {
     if (!n || !x || !y || B <= 0 || H <= 0 || W <= 0) return DNS2D_ERR_ARG;
@@ -3110,6 +3129,7 @@ extern "C" int dns2d_cnn_forward(dns2d_cnn *n, const float *x, int B, int H, int
     rc = cnn_forward_dev(n, B, H, W);
     if (rc) return rc;
     CNN_CUDA(cudaMemcpyAsync(y, n->z[n->layers - 1], (size_t)B * H * W * 4, cudaMemcpyDeviceToHost, n->stream), "out copy");
+    if (n->train_tc) return train_tc_status(n);
     CNN_CUDA(cudaStreamSynchronize(n->stream), "forward sync");
     return DNS2D_OK;
 }
@@ -3148,18 +3168,6 @@ extern "C" int dns2d_cnn_set_train_tc(dns2d_cnn *n, int on)
     if (on && n->channels > dns2d::cnngemm::BN)
         return nfail(n, DNS2D_ERR_SIZE, "tensor-core training needs at most 32 channels");
     n->train_tc = on;
-    return DNS2D_OK;
-}
-
-// the tensor-core training GEMMs' wait flag (0 when no GEMM ran); the stream is synchronised
-static int train_tc_status(dns2d_cnn *n)
-{
-    int flag[2] = {0, 0};
-    if (n->gw.err) CNN_CUDA(cudaMemcpyAsync(flag, n->gw.err, 4, cudaMemcpyDeviceToHost, n->stream), "flag copy");
-    if (n->planes.err)
-        CNN_CUDA(cudaMemcpyAsync(flag + 1, n->planes.err, 4, cudaMemcpyDeviceToHost, n->stream), "flag copy");
-    CNN_CUDA(cudaStreamSynchronize(n->stream), "flag sync");
-    if (flag[0] || flag[1]) return nfail(n, DNS2D_ERR_TIMEOUT, "tensor-core training GEMM wait timed out");
     return DNS2D_OK;
 }
 
@@ -3237,6 +3245,8 @@ extern "C" int dns2d_cnn_train(dns2d_cnn *n, int iters, int batch, float lr, uin
     const int H = n->data_H, W = n->data_W;
     int rc = cnn_reserve(n, batch, H, W);
     if (rc) return rc;
+    const long long step0 = n->step;
+    CNN_CUDA(cudaMemsetAsync(n->adam_steps, 0, sizeof(int), n->stream), "step count clear");
     uint64_t st = seed;
     std::vector<int> idx((size_t)n->data_n);
     const size_t xs = (size_t)3 * H * W, ts = (size_t)H * W;
@@ -3264,13 +3274,21 @@ extern "C" int dns2d_cnn_train(dns2d_cnn *n, int iters, int batch, float lr, uin
         const float c1 = 1.0f - (float)std::pow((double)b1, (double)n->step);
         const float c2 = 1.0f - (float)std::pow((double)b2, (double)n->step);
         dns2d::cnn::k_adam<<<64, 256, 0, n->stream>>>(n->params, n->grad, n->adam_m, n->adam_v, n->nparams, lr, b1, b2,
-                                                      1e-8f, c1, c2);
+                                                      1e-8f, c1, c2, n->train_tc ? n->gw.err : nullptr,
+                                                      n->train_tc ? n->planes.err : nullptr, n->adam_steps);
         CNN_CUDA(cudaGetLastError(), "adam");
         if (losses) losses[it] = loss;
     }
     CNN_CUDA(cudaStreamSynchronize(n->stream), "train sync");
     n->gen += 1;
-    return train_tc_status(n);
+    rc = train_tc_status(n);
+    if (rc == DNS2D_ERR_TIMEOUT) {  // the iterations from the failed one on were not applied
+        int applied = 0;
+        CNN_CUDA(cudaMemcpyAsync(&applied, n->adam_steps, sizeof(int), cudaMemcpyDeviceToHost, n->stream), "step count copy");
+        CNN_CUDA(cudaStreamSynchronize(n->stream), "step count sync");
+        n->step = step0 + applied;
+    }
+    return rc;
 }
 
 // ============================================================================================
