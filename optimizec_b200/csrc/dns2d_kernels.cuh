@@ -536,15 +536,15 @@ struct TwCat {
     static constexpr int off(int R, int NS, int outer = 0) { return cat.find(R, NS, outer); }
 };
 
-// Inverse x transform of a row pair on the large-grid plan: the half spectra A = U[k], B = W[k]
-// (k < H, consecutive k KS float2 apart) of two real rows a, b are packed
+// Inverse x transform of a row pair on the large-grid plan: the half spectra A, B of two real rows a, b
+// lie side by side, 16 bytes per mode k < H (AB + k KS, one load), and are packed
 // Hermitian-wise as A + iB and transformed (C2R semantics: only Re of the k = 0 entries is used).
 // Thread j < L/R3 is left holding v[q] = (a(x), b(x)) at x = j + q L/R3; the last inverse stage
 // runs in registers.  Used by NEXTDT (rows u, w of one physical row, for the CFL maximum) and
 // OM2PHYS (two physical rows of one field).
 template <int N, int KS>
-__device__ __forceinline__ void rows_inverse2(const float2 *__restrict__ U, const float2 *__restrict__ W, float2 *s,
-                                              const float2 *__restrict__ tw, float2 (&v)[Cfg2<N>::R3])
+__device__ __forceinline__ void rows_inverse2(const float2 *__restrict__ AB, float2 *s, const float2 *__restrict__ tw,
+                                              float2 (&v)[Cfg2<N>::R3])
 {
     using C = Cfg2<N>;
     constexpr int L = C::L, H = C::H, R1 = C::R1, R2 = C::R2, R3 = C::R3, PS = C::PS;
@@ -567,8 +567,9 @@ __device__ __forceinline__ void rows_inverse2(const float2 *__restrict__ U, cons
             b[r] = a[r];
             const int k = jb + r * LR1;
             if (!slot_in_band<L, R1, H, L - H>(r) && r * LR1 < H && k < H) {
-                a[r] = U[(size_t)k * KS];
-                b[r] = W[(size_t)k * KS];
+                const float4 ab = *reinterpret_cast<const float4 *>(AB + (size_t)k * KS);
+                a[r] = make_float2(ab.x, ab.y);
+                b[r] = make_float2(ab.z, ab.w);
             }
         }
         float2 v[R1];
@@ -669,7 +670,7 @@ __global__ void __launch_bounds__(Cfg2<N>::NT, 3) k_rows_velocity2(Pointers p0, 
     __shared__ float red[32];
     const int z = blockIdx.x, j = threadIdx.x;
     float2 v[R3];
-    rows_inverse2<N, widx_kx_stride>(p.work + widx<L, H>(0, z, 0), p.work + widx<L, H>(1, z, 0), s, p.tw, v);
+    rows_inverse2<N, widx_kx_stride>(p.work + widx<L, H>(0, z, 0), s, p.tw, v);
     float m = 0.0f;
     if (j < LR3) {
 #pragma unroll
@@ -736,7 +737,7 @@ __global__ void __launch_bounds__(Cfg2<N>::NT, 3) k_rows_pair2(Pointers p, const
     __shared__ float red[32];
     const int z = 2 * blockIdx.x, j = threadIdx.x;
     float2 v[R3];
-    rows_inverse2<N, sidx_kx_stride>(scratch + widx1<L, H>(z, 0), scratch + widx1<L, H>(z + 1, 0), s, p.tw, v);
+    rows_inverse2<N, sidx_kx_stride>(scratch + widx1<L, H>(z, 0), s, p.tw, v);
     float mn = 3.402823466e38f, mx = -3.402823466e38f;
     if (j < LR3) {
 #pragma unroll
