@@ -9,6 +9,8 @@
 #pragma once
 #include "cnn_math.cuh"
 
+#include <type_traits>
+
 namespace dns2d {
 namespace cnn {
 
@@ -84,7 +86,7 @@ __global__ void __launch_bounds__(kConvThreads) k_conv3x3(const float *__restric
     const int tiles_x = (W + kConvCols - 1) / kConvCols;
     const int x0 = (blockIdx.x % tiles_x) * kConvCols, y0 = (blockIdx.x / tiles_x) * TR;
     const int co0 = blockIdx.y * NCO, b = blockIdx.z;
-    const int px = (pg & 3) * 4, py = pg >> 2;
+    const int px = (pg & 3) * 4, py = pg >> 2, oy = y0 + py, ox = x0 + px;
     const float *xb = x + (size_t)b * Ci * H * W;
     float2 acc[4][4];
 #pragma unroll
@@ -92,15 +94,12 @@ __global__ void __launch_bounds__(kConvThreads) k_conv3x3(const float *__restric
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[p][j] = make_float2(0.f, 0.f);
     float *tin = sm, *tw = sm + kConvCi * (TR + 2) * kConvPitch;  // [ci][TR + 2][pitch], [ci][tap][NCO]
-    for (int c0 = 0; c0 < Ci; c0 += kConvCi) {
-        const int nc = min(kConvCi, Ci - c0);
-        if (c0 > 0) __syncthreads();
-        for (int e = tid; e < nc * 9 * (NCO / 4); e += kConvThreads) {
-            const int r = e / (NCO / 4), q = (e % (NCO / 4)) * 4;
-            cp_async16f(tw + r * NCO + q, w + (size_t)(c0 * 9 + r) * NP + co0 + q);
-        }
-        for (int e = tid; e < nc * (TR + 2) * (kConvCols + 2); e += kConvThreads) {
-            const int ci = e / ((TR + 2) * (kConvCols + 2)), r = e - ci * (TR + 2) * (kConvCols + 2);
+    // the tile's rows of nc channels; a last tile that reaches beyond the image takes the image's rows only
+    // (16 rows, 8 channels, one CTA: 14.7 -> 13.0 us)
+    auto load_rows = [&](int c0, int nc, auto whole) {
+        const int per = (decltype(whole)::value ? TR + 2 : H - y0 + 2) * (kConvCols + 2);
+        for (int e = tid; e < nc * per; e += kConvThreads) {
+            const int ci = e / per, r = e - ci * per;
             const int ry = r / (kConvCols + 2), rx = r - ry * (kConvCols + 2);
             int yy = y0 + ry - 1, xx = x0 + rx - 1;  // periodic; tiles may reach beyond the image
             if (yy < 0) yy += H;
@@ -109,9 +108,19 @@ __global__ void __launch_bounds__(kConvThreads) k_conv3x3(const float *__restric
             while (xx >= W) xx -= W;
             cp_async4(tin + (ci * (TR + 2) + ry) * kConvPitch + rx, xb + ((size_t)(c0 + ci) * H + yy) * W + xx);
         }
+    };
+    for (int c0 = 0; c0 < Ci; c0 += kConvCi) {
+        const int nc = min(kConvCi, Ci - c0);
+        if (c0 > 0) __syncthreads();
+        for (int e = tid; e < nc * 9 * (NCO / 4); e += kConvThreads) {
+            const int r = e / (NCO / 4), q = (e % (NCO / 4)) * 4;
+            cp_async16f(tw + r * NCO + q, w + (size_t)(c0 * 9 + r) * NP + co0 + q);
+        }
+        if (y0 + TR <= H) load_rows(c0, nc, std::true_type{});
+        else load_rows(c0, nc, std::false_type{});
         cp_async_all();
         __syncthreads();
-        for (int ci = 0; ci < nc; ++ci) {
+        for (int ci = 0; ci < nc && oy < H; ++ci) {
             const float *ti = tin + (ci * (TR + 2) + py) * kConvPitch + px;
             const float *wi = tw + ci * 9 * NCO + cg * 8;
 #pragma unroll
@@ -135,7 +144,6 @@ __global__ void __launch_bounds__(kConvThreads) k_conv3x3(const float *__restric
             }
         }
     }
-    const int oy = y0 + py, ox = x0 + px;
     if (oy >= H || ox >= W) return;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -320,6 +328,47 @@ __global__ void __launch_bounds__(256) k_wgrad_reduce(const float *__restrict__ 
     if (threadIdx.x >= 32 || co >= Co) return;
     if (tap == 9) db[co] = (float)s;
     else dw[((size_t)co * Ci + ci) * 9 + tap] = (float)s;
+}
+
+// The same for few pixels and channels: a CTA per (ci, co) over all pixels, one launch.  Two launches and the
+// latency of a CTA's first pieces bound the kernels above there: 10.4 us at 16^2, 8 x 8 channels, where this
+// one takes 5.2.  wgrad_pairs: where it is the faster one (measured, this against those, in us, at B H W pixels
+// and Ci x Co channels: 2304 and 16 x 16 12.1 / 14.5, 4096 18.5 / 16.2; 576 and 32 x 32 11.9 / 12.5, 1152
+// 17.4 / 12.8; 64 and 64 x 64 17.6 / 12.1).
+constexpr bool wgrad_pairs(long long pixels, int Ci, int Co)
+{
+    return pixels <= 2048 && Ci * Co <= 1024 && pixels * Ci * Co <= 1 << 19;
+}
+__global__ void __launch_bounds__(256) k_wgrad_pairs(const float *__restrict__ x, const float *__restrict__ dy,
+                                                     float *__restrict__ dw, float *__restrict__ db, int B, int Ci, int Co,
+                                                     int H, int W)
+{
+    __shared__ float red[10][256];
+    const int ci = blockIdx.x, co = blockIdx.y, HW = H * W;
+    float acc[10];  // 9 taps, db
+#pragma unroll
+    for (int k = 0; k < 10; ++k) acc[k] = 0.0f;
+    for (int p = threadIdx.x; p < B * HW; p += 256) {
+        const int b = p / HW, r = p - b * HW, yy = r / W, xx = r - yy * W;
+        const int sy[3] = {(yy == 0 ? H - 1 : yy - 1) * W, yy * W, (yy == H - 1 ? 0 : yy + 1) * W};
+        const int sx[3] = {xx == 0 ? W - 1 : xx - 1, xx, xx == W - 1 ? 0 : xx + 1};
+        const float g = __ldg(dy + ((size_t)b * Co + co) * HW + r);
+        const float *xc = x + ((size_t)b * Ci + ci) * HW;
+#pragma unroll
+        for (int k = 0; k < 9; ++k) acc[k] = fmaf(g, __ldg(xc + sy[k / 3] + sx[k % 3]), acc[k]);
+        acc[9] += g;
+    }
+#pragma unroll
+    for (int k = 0; k < 10; ++k) red[k][threadIdx.x] = acc[k];
+    __syncthreads();
+    for (int o = 128; o > 0; o >>= 1) {
+        if ((int)threadIdx.x < o)
+#pragma unroll
+            for (int k = 0; k < 10; ++k) red[k][threadIdx.x] += red[k][threadIdx.x + o];
+        __syncthreads();
+    }
+    if (threadIdx.x < 9) dw[((size_t)co * Ci + ci) * 9 + threadIdx.x] = red[threadIdx.x][0];
+    if (threadIdx.x == 9 && ci == 0) db[co] = red[9][0];
 }
 
 // one minibatch from the resident data set: sample src[blockIdx.y] (xs inputs, ts targets) to place

@@ -2953,16 +2953,22 @@ int cnn_backward_dev(dns2d_cnn *n, int B, int H, int W)
         }
         return DNS2D_OK;
     }
-    pack_fp32(n, n->stream);  // a forward in tensor-core mode leaves them unpacked
+    if (n->train_tc) pack_fp32(n, n->stream);  // the forward ran as GEMMs; in FP32 it has packed them
     for (int l = n->layers - 1; l >= 0; --l) {
         const float *xin = (l == 0) ? n->xin : n->a[l - 1];
         float *dw = n->grad + n->woff[l];
         float *db = dw + (size_t)n->co[l] * n->ci[l] * 9;
-        const int tiles = ((n->ci[l] + 31) / 32) * ((n->co[l] + 31) / 32);
-        const int G = wgrad_ctas(tiles, (long long)B * H * ((W + dns2d::cnn::kWgCols - 1) / dns2d::cnn::kWgCols));
-        dns2d::cnn::k_conv3x3_wgrad<<<dim3(G, tiles), dns2d::cnn::kWgThreads, dns2d::cnn::wgrad_smem(), n->stream>>>(
-            xin, dz, n->wg_part, B, n->ci[l], n->co[l], H, W);
-        dns2d::cnn::k_wgrad_reduce<<<dim3(9 * 32 + 1, tiles), 256, 0, n->stream>>>(n->wg_part, G, dw, db, n->ci[l], n->co[l]);
+        if (dns2d::cnn::wgrad_pairs((long long)B * H * W, n->ci[l], n->co[l])) {
+            dns2d::cnn::k_wgrad_pairs<<<dim3(n->ci[l], n->co[l]), 256, 0, n->stream>>>(xin, dz, dw, db, B, n->ci[l],
+                                                                                     n->co[l], H, W);
+        } else {
+            const int tiles = ((n->ci[l] + 31) / 32) * ((n->co[l] + 31) / 32);
+            const int G = wgrad_ctas(tiles, (long long)B * H * ((W + dns2d::cnn::kWgCols - 1) / dns2d::cnn::kWgCols));
+            dns2d::cnn::k_conv3x3_wgrad<<<dim3(G, tiles), dns2d::cnn::kWgThreads, dns2d::cnn::wgrad_smem(), n->stream>>>(
+                xin, dz, n->wg_part, B, n->ci[l], n->co[l], H, W);
+            dns2d::cnn::k_wgrad_reduce<<<dim3(9 * 32 + 1, tiles), 256, 0, n->stream>>>(n->wg_part, G, dw, db, n->ci[l],
+                                                                                     n->co[l]);
+        }
         if (l > 0) {
             conv(dz, n->wpack + n->pk_bwd[l], nullptr, n->z[l - 1], other, nullptr, B, n->co[l], n->ci[l], H, W, n->stream);
             std::swap(dz, other);
