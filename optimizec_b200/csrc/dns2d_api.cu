@@ -2618,7 +2618,7 @@ struct dns2d_cnn {
     float *params = nullptr, *grad = nullptr, *adam_m = nullptr, *adam_v = nullptr;
     std::vector<float *> z, a;     // pre-activations / activations per layer (capacity cap_elems each)
     float *xin = nullptr, *tgt = nullptr, *gout = nullptr, *gtmp = nullptr;
-    float *wg_part = nullptr;      // partial sums of the FP32 weight gradient
+    float *wg_part = nullptr;      // partial sums of the FP32 weight gradient, allocated by its first use
     float *wpack = nullptr;        // packed weights of the FP32 convolutions, per layer forward and data gradient
     std::vector<size_t> pk_fwd, pk_bwd;
     size_t cap_elems = 0;          // per activation tensor: B * max(C, 3) * H * W
@@ -2626,7 +2626,7 @@ struct dns2d_cnn {
     int capB = 0, capH = 0, capW = 0;
     double *part = nullptr;
     long long step = 0;
-    int *adam_steps = nullptr;     // iterations that the current dns2d_cnn_train has applied
+    int *adam_steps = nullptr;     // iterations that the current dns2d_cnn_train has applied (behind part)
     float *data_x = nullptr, *data_t = nullptr;  // device-resident training set
     int data_n = 0, data_H = 0, data_W = 0;
     // BF16 tensor-core inference path (cnn_tc.cuh, cnn_net.cuh): packed weights, padded
@@ -2962,6 +2962,12 @@ int cnn_backward_dev(dns2d_cnn *n, int B, int H, int W)
             dns2d::cnn::k_wgrad_pairs<<<dim3(n->ci[l], n->co[l]), 256, 0, n->stream>>>(xin, dz, dw, db, B, n->ci[l],
                                                                                      n->co[l], H, W);
         } else {
+            if (!n->wg_part) {
+                // one CTA's sums per channel tile at least, two per SM in all at most
+                const size_t ct = (size_t)(n->channels + 31) / 32, ctas = std::max<size_t>(ct * ct, 148 * dns2d::cnn::kWgCtas);
+                CNN_CUDA(cudaMalloc((void **)&n->wg_part, ctas * dns2d::cnn::kWgPart * sizeof(float)),
+                         "weight gradient partials alloc");
+            }
             const int tiles = ((n->ci[l] + 31) / 32) * ((n->co[l] + 31) / 32);
             const int G = wgrad_ctas(tiles, (long long)B * H * ((W + dns2d::cnn::kWgCols - 1) / dns2d::cnn::kWgCols));
             dns2d::cnn::k_conv3x3_wgrad<<<dim3(G, tiles), dns2d::cnn::kWgThreads, dns2d::cnn::wgrad_smem(), n->stream>>>(
@@ -3013,7 +3019,6 @@ extern "C" void dns2d_cnn_destroy(dns2d_cnn *n)
     cudaFree(n->gout);
     cudaFree(n->gtmp);
     cudaFree(n->part);
-    cudaFree(n->adam_steps);
     cudaFree(n->data_x);
     cudaFree(n->data_t);
     cudaFree(n->wtc);
@@ -3071,14 +3076,12 @@ extern "C" int dns2d_cnn_create(dns2d_cnn **out, int layers, int channels, uint6
         n->pk_bwd.push_back(pk);
         pk += (size_t)n->co[l] * 9 * dns2d::cnn::packed_channels(n->ci[l]);
     }
-    const int ct = (channels + 31) / 32, tiles = ct * ct;
-    const size_t wg = (size_t)tiles * wgrad_ctas(tiles, 1ll << 30) * dns2d::cnn::kWgPart;
     if (cudaMalloc((void **)&n->params, off * 4) != cudaSuccess || cudaMalloc((void **)&n->grad, off * 4) != cudaSuccess ||
         cudaMalloc((void **)&n->adam_m, off * 4) != cudaSuccess || cudaMalloc((void **)&n->adam_v, off * 4) != cudaSuccess ||
-        cudaMalloc((void **)&n->wg_part, std::max(wg, (size_t)148 * dns2d::cnn::kWgCtas * dns2d::cnn::kWgPart) * 4) != cudaSuccess ||
-        cudaMalloc((void **)&n->wpack, pk * 4) != cudaSuccess || cudaMalloc((void **)&n->part, 256 * 8) != cudaSuccess ||
-        cudaMalloc((void **)&n->adam_steps, sizeof(int)) != cudaSuccess)
+        cudaMalloc((void **)&n->wpack, pk * 4) != cudaSuccess ||
+        cudaMalloc((void **)&n->part, 256 * sizeof(double) + sizeof(int)) != cudaSuccess)
         return bail(DNS2D_ERR_NOMEM);
+    n->adam_steps = reinterpret_cast<int *>(n->part + 256);
     if (cudaMemcpy(n->params, p.data(), off * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemset(n->adam_m, 0, off * 4) != cudaSuccess || cudaMemset(n->adam_v, 0, off * 4) != cudaSuccess)
         return bail(DNS2D_ERR_CUDA);
