@@ -332,9 +332,10 @@ __global__ void __launch_bounds__(256) k_wgrad_reduce(const float *__restrict__ 
 
 // The same for few pixels and channels: a CTA per (ci, co) over all pixels, one launch.  Two launches and the
 // latency of a CTA's first pieces bound the kernels above there: 10.4 us at 16^2, 8 x 8 channels, where this
-// one takes 5.2.  wgrad_pairs: where it is the faster one (measured, this against those, in us, at B H W pixels
+// one takes 4.8.  wgrad_pairs: where it is the faster one (measured, this against those, in us, at B H W pixels
 // and Ci x Co channels: 2304 and 16 x 16 12.1 / 14.5, 4096 18.5 / 16.2; 576 and 32 x 32 11.9 / 12.5, 1152
-// 17.4 / 12.8; 64 and 64 x 64 17.6 / 12.1).
+// 17.4 / 12.8; 64 and 64 x 64 17.6 / 12.1; with the threads' sums as an FP32 tree of eight barriers, 0.4 more
+// than in FP64 behind one).
 constexpr bool wgrad_pairs(long long pixels, int Ci, int Co)
 {
     return pixels <= 2048 && Ci * Co <= 1024 && pixels * Ci * Co <= 1 << 19;
@@ -361,14 +362,16 @@ __global__ void __launch_bounds__(256) k_wgrad_pairs(const float *__restrict__ x
 #pragma unroll
     for (int k = 0; k < 10; ++k) red[k][threadIdx.x] = acc[k];
     __syncthreads();
-    for (int o = 128; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o)
+    // the threads' sums in FP64 and a fixed order, one warp per tap
+    const int lane = threadIdx.x & 31;
+    for (int k = threadIdx.x >> 5; k < 10; k += 8) {
+        double s = 0.0;
 #pragma unroll
-            for (int k = 0; k < 10; ++k) red[k][threadIdx.x] += red[k][threadIdx.x + o];
-        __syncthreads();
+        for (int i = 0; i < 8; ++i) s += (double)red[k][i * 32 + lane];
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0 && k < 9) dw[((size_t)co * Ci + ci) * 9 + k] = (float)s;
+        if (lane == 0 && k == 9 && ci == 0) db[co] = (float)s;
     }
-    if (threadIdx.x < 9) dw[((size_t)co * Ci + ci) * 9 + threadIdx.x] = red[threadIdx.x][0];
-    if (threadIdx.x == 9 && ci == 0) db[co] = red[9][0];
 }
 
 // one minibatch from the resident data set: sample src[blockIdx.y] (xs inputs, ts targets) to place

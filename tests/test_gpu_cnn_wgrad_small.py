@@ -41,3 +41,18 @@ def test_loss_and_gradients_match_oracle(layers, ch, H, W, B):
         off += n + co
     assert np.linalg.norm(g - g_ref) <= 1e-5 * np.linalg.norm(g_ref)
     np.testing.assert_array_equal(g, g2)
+
+
+def test_sums_over_threads_lose_nothing():
+    """One pixel per thread, so every sum of the one-launch kernel is over threads only, in FP64: with all
+    weights zero the output is 0, dout = -2 t / 256 and the last bias gradient is its exact sum.  In FP32 the 1
+    is lost beside 2^25."""
+    import optimizec_b200 as P
+
+    net = P.CNN(2, 1, seed=1)
+    net.set_params(np.zeros(net.num_params(), dtype=np.float32))
+    t = np.zeros((1, 1, 16, 16), dtype=np.float32)
+    t.flat[0], t.flat[1], t.flat[128] = 2.0 ** 25, -2.0 ** 25, 1.0
+    _, g = net.loss_grad(np.ones((1, 3, 16, 16), dtype=np.float32), t)
+    net.close()
+    assert g[-1] == -2.0 / 256
