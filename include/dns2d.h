@@ -14,6 +14,13 @@
  *   phys   physical planes [L][L] float32, x fastest: comp 0 = u, 1 = w, 2 = scalar (omega,
  *          stream function or |u| after the matching call)
  * A state owns one CUDA stream; calls on one state must come from one host thread.
+ *
+ * Rounding: the same calls give the same fields bit for bit, run after run.  With the default
+ * configuration of a size this also holds from one build of the library to the next, so that a run
+ * repeated or continued (restart.bin) with a later build can be compared mode by mode; a size that a
+ * build rounds otherwise is listed here (N = 1024 since its in-place passes: relative L2 7e-7 after a
+ * short run).  A tuned radix plan (dns2d_autotune) rounds otherwise than the default one, and networks
+ * (dns2d_cnn_*, closed runs) are not covered from build to build.
  */
 #ifndef DNS2D_H
 #define DNS2D_H
@@ -225,7 +232,8 @@ int dns2d_cnn_loss_grad(dns2d_cnn *n, const float *x, const float *t, int B, int
 int dns2d_cnn_set_dataset(dns2d_cnn *n, const float *x, const float *t, int count, int H, int W);
 int dns2d_cnn_train(dns2d_cnn *n, int iters, int batch, float lr, uint64_t seed, double *losses);
 /* Training convolutions on the tensor cores (off by default; channels <= 32): forward, data and
- * weight gradients as tcgen05 GEMMs over bf16 im2col expansions with FP32 accumulation (the
+ * weight gradients as tcgen05 GEMMs with bf16 operands and FP32 accumulation, read from bf16 chunk
+ * planes where W is a multiple of 16 and channels >= 4, else from im2col expansions (the
  * weight gradient split over the pixels, partials summed in fixed order in FP64); loss, GELU and
  * Adam stay FP32.  Applies to dns2d_cnn_forward, dns2d_cnn_loss_grad and dns2d_cnn_train; the
  * gradients then agree with the FP32 ones to bf16 rounding of the operands. */

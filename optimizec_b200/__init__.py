@@ -227,7 +227,8 @@ def autotune(N: int, device: int = 0) -> dict:
 
 def set_tuning(N: int, rows_tile=0, cols_groups=0, pf_rows=296, pf_cols=74, plan_rows=0, plan_cols=0,
                device: int = 0):
-    """Pin the kernel configuration of size N (dns2d_set_tuning)."""
+    """Pin the kernel configuration of size N (dns2d_set_tuning).  rows_tile and the plans select kernels of
+    N <= 512; cols_groups, pf_rows and pf_cols are accepted and reported, and no kernel reads them."""
     cfg = (C.c_int * 6)(rows_tile, cols_groups, pf_rows, pf_cols, plan_rows, plan_cols)
     rc = lib().dns2d_set_tuning(N, device, cfg)
     if rc:

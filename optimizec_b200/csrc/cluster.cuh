@@ -75,7 +75,7 @@ constexpr TwCatalog make_catalog_c()
 template <int N>
 struct TwCatC {
     static constexpr TwCatalog cat = make_catalog_c<N>();
-    static constexpr int off(int R, int NS, int outer = 0) { return cat.find(R, NS, outer); }
+    static constexpr int off(int R, int NS) { return cat.find(R, NS, 0); }
 };
 
 // W_L^{r m} (forward sign) from the cross stage table, r = 1..3

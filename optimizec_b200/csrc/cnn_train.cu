@@ -151,9 +151,10 @@ constexpr int kConvStages = 3, kConvCtas = 2;  // 4 stages leave one CTA per SM:
 constexpr int kConvThreads = 320;  // warps 0-7 epilogue, 8 producer, 9 MMA issuer
 
 // One convolution over planes (forward or data gradient).  CTA c takes tiles c, c + G, ...  At 384^2,
-// batch 4, 32 channels (B200): 57 us; the chain of a tile's 18 MMAs alone takes 36 (the tensor pipe is
-// busy half of that), the epilogue's erf and stores the rest (issue 54 % busy); the tensors moved (z, planes
-// in and out, 150 MB) would take 23.  Against 97 us of im2col expansion and 88 us of GEMM before.  Two CTAs per SM give 16 epilogue warps.
+// batch 4, 32 channels (B200): 57 us forward, 62 for a data gradient.  Bound by the epilogue's erf and stores
+// (issue 68-70 % busy); without them (one output channel, no GELU) the chain of a tile's 18 dependent MMAs
+// alone takes 36 (tensor pipe 15 % busy); the tensors moved (z, planes in and out, 150 MB) would take 23.
+// Against 97 us of im2col expansion and 88 us of GEMM before.  Two CTAs per SM give 16 epilogue warps.
 // Every wait is bounded (2 s): one that runs out sets *err, and each role ends after the copies and
 // MMAs in flight.
 __global__ void __launch_bounds__(kConvThreads, kConvCtas) k_conv_planes(const __grid_constant__ ConvArgs q)
@@ -336,7 +337,7 @@ __host__ __device__ constexpr int wgrad_planes(int rows, int nchi, int ncho) { r
 // dx pixels further on.  Accumulator dx: row m = (dy nchi + chunk) 8 + channel, row 8 x planes the
 // product with a plane of ones (db).  The M tile's 16 planes reach beyond those into whatever lies
 // behind them in shared memory: those rows are not read.  CTA c takes items c, c + G, ... into
-// accumulators that it writes once: part[c].  Measured 68 us at 384^2, batch 4, 32 channels against
+// accumulators that it writes once: part[c].  Measured 63 us at 384^2, batch 4, 32 channels against
 // 0.41 ms of expansion, packing and GEMM before; bound by the chain of MMAs on an accumulator (252 of
 // them, about 290 cycles apart when none lies between), whose grouping fixes the rounding of the sums.
 // Waits are bounded as in k_conv_planes.

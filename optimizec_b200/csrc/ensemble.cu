@@ -89,7 +89,8 @@ __device__ __forceinline__ void ens_cols(const Pointers &p, int item, int first,
     const int tid = opaque_tid();  // nothing of it hoisted out of the work loop
     constexpr int L = C::L, H = C::H, LP = C::LP, NT = kEnsThreads, CG = ens_cols_per_item<N>(), B = 2 * CG;
     const int kx0 = item * CG;
-    // (z, kx0 + c) for c < CG and z%4 are CG * 4 consecutive float2 of a 4-row tile: read them so
+    // both components of (z, kx0 + c), c < CG and z % 4, are CG * 8 consecutive float2 of a 4-row tile: a warp
+    // reads every other one of them, then the others
     for (int e = tid; e < CG * L; e += NT) {
         const int z4 = e / (CG * 4), rem = e - z4 * (CG * 4), c = rem >> 2, z = 4 * z4 + (rem & 3);
         smem[(2 * c) * LP + sidx<PS>(z)] = __ldcg(p.work + widx<L, H>(0, z, kx0 + c));

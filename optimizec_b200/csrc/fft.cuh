@@ -107,7 +107,10 @@ __device__ __forceinline__ float2 cfma_mi(float2 t, float f, float2 m)
 //
 // Which of its two products an FMA rounds is fixed here so that the results equal, bit for bit, those of
 // the scalar expression (a.x c - a.y s, a.x s + a.y c) as the compiler contracts it: the real part keeps
-// a.x c exact, the imaginary part a.x s, or (ALT) a.y c where the sum is written as a difference.
+// a.x c exact, the imaginary part a.x s, or (ALT) a.y c where the sum is written as a difference.  Which
+// rotations take ALT was found by comparison with nvcc 12.9's scalar code, not derived: tests/fft_codelets.cu
+// compares the packed forms with the scalar one (cscalar) bit for bit, so a compiler that contracts otherwise
+// shows there.
 template <bool ALT = false>
 __device__ __forceinline__ float2 crot(float2 a, float c, float s)
 {

@@ -23,17 +23,19 @@
 // Rounding: both transforms compute node by node what auto-sort plans do (decimation in time: twiddles
 // before a butterfly), and the packed operations round where the scalar expressions of those plans round
 // (fft.cuh), so that with the plans (16, 12, 16) and (16, 24, 16), the same in both directions, N = 2048
-// and 4096 have the auto-sort kernels' results bit for bit.  It matters: FP32 rounding of the products, times
-// k^2, is 1e-3 of the field's RMS in single modes of the corners, and a run compared with an earlier one
-// would show it.  A first transform by decimation in frequency (twiddles after a butterfly, fetched once)
-// was 1-9 % faster (N = 4096 386 us per step, 2048 89.7; with decimation in time 392, 98), N = 8192 / 9216 on three-stage in-place
-// passes twice as fast as the clusters (1.75 / 2.55 ms), N = 512 and 256 15.3 and 10.6 us (20.6 and 12.1) and the
-// 64-member ensemble 77 us per step (125): all with other rounding, further from an earlier run than two runs may be.
+// and 4096 have the auto-sort kernels' results bit for bit: the default configuration of a size keeps its
+// rounding from build to build (dns2d.h), so that runs and restarts can be compared across builds mode by
+// mode.  FP32 rounding of the products, times k^2, is 1e-3 of the field's RMS in single modes of the corners.
+// Measured with other rounding and not kept for that reason alone: a first transform by decimation in
+// frequency (twiddles after a butterfly, fetched once; N = 4096 386 us per step where decimation in time
+// took 392 in the same build, 2048 89.7 / 98), N = 8192 / 9216 on three-stage in-place passes (1.75 / 2.55 ms,
+// 3.44 / 4.70 on the clusters), N = 512 and 256 (15.3 and 10.6 us; 20.1 and 11.9 now) and the 64-member ensemble
+// (77 us per step; 119 now).  Auto-sort stages within one CTA could keep the rounding there; not built.
 //
 // Bounds (N = 4096 on B200, 1965 MHz; ncu): the row pass is bound by the L1 / shared-memory data
-// pipe (67-75 % of its cycles busy; 24 % before the loads' and twiddles' share fell), the column pass
-// by the latency of its phases at two CTAs per SM (HBM 35 %, issue 32 %).  Measured (rows / columns,
-// one launch): N = 4096 0.254 / 0.293 -> 0.193 / 0.201 ms, N = 2048 67.6 / 71.7 -> 52.1 / 54.7 us,
+// pipe (66 % of its cycles busy), the column pass by the latency of its phases at two CTAs per SM (HBM
+// 38 %, issue 35 %).  Measured (rows / columns, one launch): N = 4096 0.254 / 0.293 -> 0.194 / 0.200 ms,
+// N = 2048 67.6 / 71.7 -> 52.1 / 54.7 us,
 // N = 1024 27.0 / 28.2 -> 20.3 / 23.2 us against the auto-sort kernels that these replace (one row,
 // or one array and thread group, per 384 threads).
 // Tried and slower, or no faster: each sequence on its own lane with scalar butterflies (rows 0.185,
